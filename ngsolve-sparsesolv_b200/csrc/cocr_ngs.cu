@@ -252,7 +252,11 @@ static std::string pre_key(const ssv_precond* pre) {
                     std::to_string(precond_generation(pre)) + ":" + std::to_string((size_t)pre->xw.get());
     if (pre->kind == 1) {
         k += ":" + std::to_string(pre->A->dtype == SSV_F64 ? pre->ic_d.lo : pre->ic_z.lo) + ":" +
-             std::to_string(pre->A->dtype == SSV_F64 ? pre->ic_d.abmc : pre->ic_z.abmc);
+             std::to_string(pre->A->dtype == SSV_F64 ? pre->ic_d.abmc : pre->ic_z.abmc) + ":" +
+             std::to_string((size_t)pre->ic_d.sweep_f.stream.get()) + ":" +
+             std::to_string((size_t)pre->ic_d.sweep_b.stream.get()) + ":" +
+             std::to_string((size_t)pre->ic_z.sweep_f.stream.get()) + ":" +
+             std::to_string((size_t)pre->ic_z.sweep_b.stream.get());
     }
     return k;
 }
@@ -412,6 +416,7 @@ static void run_cocr_ngs(ssv_matrix* A, ssv_precond* pre, const uint8_t* fd, int
         // out of iterations, or a cycle that could not take a single step
         if (used >= maxiter || h.updates == 0 || rs < 1e-300) break;
     }
+    precond_check(pre, s);
     if (refine) {
         *iterations = used;
         if (info) {
@@ -525,6 +530,7 @@ static void run_pcg(ssv_matrix* A, ssv_precond* pre, const uint8_t* fd, const ss
     SSV_CUDA(cudaMemcpyAsync(&h, dst, sizeof(h), cudaMemcpyDeviceToHost, s));
     SSV_CUDA(cudaStreamSynchronize(s));
     if (h.status == SSV_ERR_TIMEOUT) fail(SSV_ERR_TIMEOUT, "CG loop guard fired");
+    precond_check(pre, s);
     std::memset(res, 0, sizeof(*res));
     res->converged = h.converged;
     res->iterations = h.iters;

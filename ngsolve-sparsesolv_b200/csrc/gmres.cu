@@ -187,6 +187,7 @@ static void run_gmres(ssv_matrix* A, ssv_precond* pre, const uint8_t* fd, int ma
     }
     SSV_CUDA(cudaStreamSynchronize(s));
     SSV_LAUNCH_CHECK();
+    precond_check(pre, s);
     *iterations = total;
 }
 

@@ -1,7 +1,7 @@
 // mrtr.cu -- SGS-MRTR (solvers/sgs_mrtr_solver.hpp) on the device.
 //
 // Split-formula MRTR on D A D (D = |diag A|^{-1/2}) with level-scheduled
-// forward / backward sweeps over L = lower(D A D). Per iteration:
+// forward / backward sweeps over L = lower(D A D) (sweep.cuh). Per iteration:
 // backward sweep, forward sweep on (rd - u), one fused pass that forms
 // Ard = L^{-1}(rd-u) + u and the three inner products, and one fused update
 // pass with the residual norm; the scalar recurrences (zeta, eta, nu) run on
@@ -212,6 +212,10 @@ struct MrtrPattern {
     DevBuf<int> Lrp, Lci, Lsrc, Urp, Uci, Usrc, rows_f, rows_b;
     DevBuf<S> Lv, Uv, u, Ard, y, rd;
     DevBuf<double> D, iD;
+    // both sweeps in one launch each (else level by level)
+    Sweep<S> sweep_f, sweep_b;
+    bool diag = false;  // every row has its diagonal entry
+    bool swept() const { return diag && sweep_f.ready && sweep_b.ready; }
 };
 
 template <typename S> MrtrPattern<S>& mrtr_of(ssv_solver* s);
@@ -274,10 +278,14 @@ void run_mrtr(ssv_solver* sv, const ssv_config& cfg, const S* d_b, S* d_x, ssv_r
         group_by_level(lev, nl, rws, off);
         P.rows_f.upload(rws.data(), rws.size(), s);
         for (int l = 0; l < nl; ++l) P.fwd.push_back({off[l], off[l + 1]});
+        P.diag = true;
+        for (int i = 0; i < n && P.diag; ++i) P.diag = lrp[i] < lrp[i + 1] && lci[lrp[i + 1] - 1] == i;
+        if (P.diag) P.sweep_f.build(n, lrp, lci, true, rws, off, s);
         nl = build_levels(n, urp.data(), uci.data(), true, lev);
         group_by_level(lev, nl, rws, off);
         P.rows_b.upload(rws.data(), rws.size(), s);
         for (int l = 0; l < nl; ++l) P.bwd.push_back({off[l], off[l + 1]});
+        if (P.diag && P.sweep_f.ready) P.sweep_b.build(n, urp, uci, false, rws, off, s);
         P.Lrp.upload(lrp.data(), lrp.size(), s);
         P.Lci.upload(lci.data(), lci.size(), s);
         P.Lsrc.upload(lsrc.data(), lsrc.size(), s);
@@ -301,6 +309,10 @@ void run_mrtr(ssv_solver* sv, const ssv_config& cfg, const S* d_b, S* d_x, ssv_r
     k_gather_values<S><<<grid_for(P.Usrc.size(), kBlock), kBlock, 0, s>>>((int64_t)P.Usrc.size(), P.Usrc.get(),
                                                                          P.Lv.get(), P.Uv.get());
     SSV_LAUNCH_CHECK();
+    if (P.swept()) {
+        P.sweep_f.fill(SW_DIV, P.Lrp.get(), P.Lci.get(), P.Lv.get(), SD_LAST, nullptr, nullptr, false, s);
+        P.sweep_b.fill(SW_DIV, P.Urp.get(), P.Uci.get(), P.Uv.get(), SD_FIRST, nullptr, nullptr, false, s);
+    }
     SSV_CUDA(cudaStreamSynchronize(s));
     const double t1 = wall_seconds();
     // x_mod with constrained entries zeroed, Ax = A x_mod
@@ -327,10 +339,27 @@ void run_mrtr(ssv_solver* sv, const ssv_config& cfg, const S* d_b, S* d_x, ssv_r
     if (nb2 < 1e-30) nb2 = 1.0;
 
     // rd = L^{-1} r ; y = -rd ; p = 0
-    for (const auto& lv : P.fwd)
-        k_mrtr_fwd<S><<<(lv.second - lv.first + 127) / 128, 128, 0, s>>>(lv.first, lv.second, P.rows_f.get(),
-                                                                         P.Lrp.get(), P.Lci.get(), P.Lv.get(),
-                                                                         w.r.get(), nullptr, P.rd.get(), nullptr);
+    auto forward = [&](const S* a, const S* b, S* y, KState* st) {
+        if (P.swept()) {
+            P.sweep_f.load(a, b, nullptr, st, s);
+            P.sweep_f.run(y, st, s);
+            return;
+        }
+        for (const auto& lv : P.fwd)
+            k_mrtr_fwd<S><<<(lv.second - lv.first + 127) / 128, 128, 0, s>>>(
+                lv.first, lv.second, P.rows_f.get(), P.Lrp.get(), P.Lci.get(), P.Lv.get(), a, b, y, st);
+    };
+    auto backward = [&](const S* a, S* y, KState* st) {
+        if (P.swept()) {
+            P.sweep_b.load(a, nullptr, nullptr, st, s);
+            P.sweep_b.run(y, st, s);
+            return;
+        }
+        for (const auto& lv : P.bwd)
+            k_mrtr_bwd<S><<<(lv.second - lv.first + 127) / 128, 128, 0, s>>>(
+                lv.first, lv.second, P.rows_b.get(), P.Urp.get(), P.Uci.get(), P.Uv.get(), a, y, st);
+    };
+    forward(w.r.get(), nullptr, P.rd.get(), nullptr);
     k_neg<S><<<g, kBlock, 0, s>>>(n, P.rd.get(), P.y.get());
     w.p.zero(s);
     SSV_LAUNCH_CHECK();
@@ -375,14 +404,8 @@ void run_mrtr(ssv_solver* sv, const ssv_config& cfg, const S* d_b, S* d_x, ssv_r
                             std::to_string((size_t)dst) + ";" + std::to_string((size_t)w.r.get()) + ";" +
                             std::to_string((size_t)w.partials.get()) + ";" + std::to_string(fd != nullptr);
     build_graph_loop(sv->loop, key, [&](cudaGraphConditionalHandle hc, int use_cond) {
-        for (const auto& lv : P.bwd)
-            k_mrtr_bwd<S><<<(lv.second - lv.first + 127) / 128, 128, 0, s>>>(
-                lv.first, lv.second, P.rows_b.get(), P.Urp.get(), P.Uci.get(), P.Uv.get(), P.rd.get(), P.u.get(),
-                dst);
-        for (const auto& lv : P.fwd)
-            k_mrtr_fwd<S><<<(lv.second - lv.first + 127) / 128, 128, 0, s>>>(
-                lv.first, lv.second, P.rows_f.get(), P.Lrp.get(), P.Lci.get(), P.Lv.get(), P.rd.get(), P.u.get(),
-                P.Ard.get(), dst);
+        backward(P.rd.get(), P.u.get(), dst);
+        forward(P.rd.get(), P.u.get(), P.Ard.get(), dst);
         k_mrtr_dots<S><<<g, kBlock, 0, s>>>(n, P.Ard.get(), P.u.get(), P.rd.get(), P.y.get(), dst, w.partials.get(),
                                            w.ticket.get());
         k_mrtr_update<S><<<g, kBlock, 0, s>>>(n, w.xb[0].get(), w.xb[1].get(), w.xb[2].get(), P.u.get(),
@@ -394,6 +417,7 @@ void run_mrtr(ssv_solver* sv, const ssv_config& cfg, const S* d_b, S* d_x, ssv_r
     SSV_CUDA(cudaMemcpyAsync(&h, dst, sizeof(h), cudaMemcpyDeviceToHost, s));
     SSV_CUDA(cudaStreamSynchronize(s));
     if (h.status == SSV_ERR_TIMEOUT) fail(SSV_ERR_TIMEOUT, "SGS-MRTR loop guard fired");
+    if (P.swept()) P.sweep_f.check(s);  // the sweep before the loop
     res->converged = h.converged;
     res->iterations = h.iters;
     res->final_residual = h.final_norm / h.normalizer;

@@ -9,6 +9,7 @@
 #include "host_order.hpp"
 #include "kernels.cuh"
 #include "sell.cuh"
+#include "sweep.cuh"
 
 namespace ssv {
 
@@ -228,6 +229,9 @@ struct ICDevice {
     int missing_row = -1;
     double actual_shift = 0.0;
     DevBuf<S> tw;  // forward-sweep output
+    // level schedule: both sweeps in one launch each (else level by level)
+    Sweep<S> sweep_f, sweep_b;
+    bool swept() const { return !abmc && missing_row < 0 && sweep_f.ready && sweep_b.ready; }
     // ABMC block-sweep layout (k_ic_fwd_blk / k_ic_bwd_blk): external parts of
     // L and U rows, packed strictly-lower intra-block table, diagonal
     bool blk = false;
@@ -262,6 +266,7 @@ struct ICDevice {
     void apply_fwd(const S* x, const KState* st, cudaStream_t s) const;  // x -> tw
     void apply_bwd(S* y, const KState* st, cudaStream_t s) const;        // tw -> y
     int kernels_per_apply() const {
+        if (swept()) return 3 + (scaled_apply ? 1 : 0);
         if (blk)
             return (int)fwd_cta.size() + (int)bwd_cta.size() +
                    (scaled_apply ? 1 : 0);
@@ -279,6 +284,10 @@ struct SgsDevice {
     std::vector<std::pair<int, int>> fwd_lev, bwd_lev;  // row ranges of rows_f / rows_b per level
     DevBuf<int> rows_f, rows_b;
     DevBuf<S> inv, tmp;
+    // both sweeps in one launch each (else level by level); values of vgen
+    Sweep<S> sweep_f, sweep_b;
+    unsigned vgen = 0;
+    bool swept() const { return sweep_f.ready && sweep_b.ready; }
 };
 
 }  // namespace ssv

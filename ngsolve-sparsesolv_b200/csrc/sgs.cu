@@ -3,8 +3,9 @@
 // M^{-1} = (D + U)^{-1} D (D + L)^{-1} on the FreeDofs view of A (constrained
 // rows identity, constrained columns zero), output zeroed on constrained DOFs.
 // Both sweeps run level set by level set (the reference's LevelSchedule built
-// from the full pattern, entries j < i forward and j > i backward), one
-// launch per level, one thread per row; the arithmetic of a row is the
+// from the full pattern, entries j < i forward and j > i backward), in one
+// launch each (sweep.cuh), or one launch per level with one thread per row
+// where a level or a row is too large for that; the arithmetic of a row is the
 // reference's, in its order.
 #include "objects.cuh"
 #include "solver_api.hpp"
@@ -57,14 +58,23 @@ template <typename S> SgsDevice<S>& sgs_of(ssv_precond* p);
 template <> SgsDevice<double>& sgs_of<double>(ssv_precond* p) { return p->sgs_d; }
 template <> SgsDevice<zdouble>& sgs_of<zdouble>(ssv_precond* p) { return p->sgs_z; }
 
+template <typename S>
 static void levels_of(int n, const std::vector<int>& rp, const std::vector<int>& ci, bool upper,
-                      std::vector<std::pair<int, int>>& ranges, DevBuf<int>& rows_d, cudaStream_t s) {
+                      std::vector<std::pair<int, int>>& ranges, DevBuf<int>& rows_d, Sweep<S>& sweep, cudaStream_t s) {
     std::vector<int> lev, rows, off;
     const int nl = build_levels(n, rp.data(), ci.data(), upper, lev);
     group_by_level(lev, nl, rows, off);
     ranges.clear();
     for (int l = 0; l < nl; ++l) ranges.push_back({off[l], off[l + 1]});
     rows_d.upload(rows.data(), rows.size(), s);
+    sweep.build(n, rp, ci, !upper, rows, off, s);
+}
+
+template <typename S>
+static void sgs_fill(SgsDevice<S>& g, const ssv_matrix* A, const S* v, cudaStream_t s) {
+    g.sweep_f.fill(SW_MUL, A->rp.get(), A->ci.get(), v, SD_ARRAY, g.inv.get(), g.sweep_b.pos.get(), false, s);
+    g.sweep_b.fill(SW_ICB, A->rp.get(), A->ci.get(), v, SD_ARRAY, g.inv.get(), nullptr, false, s);
+    g.vgen = A->vgen;
 }
 
 template <typename S>
@@ -82,8 +92,8 @@ static void sgs_update_t(ssv_precond* p) {
         vals = reinterpret_cast<const S*>(p->vals_bc.get());
     }
     if (!g.built) {
-        levels_of(n, A->h_rp, A->h_ci, false, g.fwd_lev, g.rows_f, s);
-        levels_of(n, A->h_rp, A->h_ci, true, g.bwd_lev, g.rows_b, s);
+        levels_of(n, A->h_rp, A->h_ci, false, g.fwd_lev, g.rows_f, g.sweep_f, s);
+        levels_of(n, A->h_rp, A->h_ci, true, g.bwd_lev, g.rows_b, g.sweep_b, s);
         g.inv.alloc(n);
         g.tmp.alloc(n);
         g.built = true;
@@ -91,6 +101,7 @@ static void sgs_update_t(ssv_precond* p) {
     }
     k_sgs_inv_diag<S><<<grid_for(n, kBlock), kBlock, 0, s>>>(n, A->rp.get(), A->ci.get(), vals, g.inv.get());
     SSV_LAUNCH_CHECK();
+    if (g.swept()) sgs_fill(g, A, vals, s);
     SSV_CUDA(cudaStreamSynchronize(s));
     p->ready = true;
 }
@@ -108,6 +119,17 @@ void sgs_apply_dev(ssv_precond* p, const S* x, S* y, const KState* st, cudaStrea
     const S* v = p->has_fd ? reinterpret_cast<const S*>(p->vals_bc.get()) : reinterpret_cast<const S*>(A->val.get());
     const int* rp = A->rp.get();
     const int* ci = A->ci.get();
+    if (g.swept()) {
+        // without a FreeDofs view the off-diagonals are the matrix's current values, as in the
+        // launches below (a solve's first application runs outside its capture and refills here)
+        if (!p->has_fd && g.vgen != A->vgen) sgs_fill(g, A, v, s);
+        g.sweep_f.load(x, nullptr, nullptr, st, s);
+        g.sweep_f.run(g.sweep_b.xs.get(), st, s);
+        g.sweep_b.run(y, st, s);
+        if (p->has_fd) launch_k(k_mask_zero<S>, grid_for(n, kBlock), kBlock, s, n, y, (const uint8_t*)p->fd.get());
+        SSV_LAUNCH_CHECK();
+        return;
+    }
     S* t = g.tmp.get();
     for (const auto& r : g.fwd_lev)
         launch_k(k_sgs_sweep<S, true>, (r.second - r.first + 127) / 128, 128, s, r.first, r.second,

@@ -236,10 +236,12 @@ void ICDevice<S>::build_pattern(int n_, const std::vector<int>& rp, const std::v
         group_by_level(lev, num_levels_f, rws, off);
         rows_f.upload(rws.data(), rws.size(), s);
         for (int l = 0; l < num_levels_f; ++l) fwd_launch.push_back({off[l], off[l + 1]});
+        sweep_f.build(n, lrp, lci, true, rws, off, s);
         num_levels_b = build_levels(n, urp.data(), uci.data(), true, lev);
         group_by_level(lev, num_levels_b, rws, off);
         rows_b.upload(rws.data(), rws.size(), s);
         for (int l = 0; l < num_levels_b; ++l) bwd_launch.push_back({off[l], off[l + 1]});
+        if (sweep_f.ready) sweep_b.build(n, urp, uci, false, rws, off, s);
     }
     // missing diagonal (ic_preconditioner.hpp:1221-1226 / :1358-1363): first
     // row in processing order whose last lower entry is not the diagonal
@@ -542,6 +544,12 @@ int ICDevice<S>::factorize(const S* vals, const ssv_config& cfg) {
         }
         SSV_LAUNCH_CHECK();
     }
+    if (swept()) {
+        // the forward sweep writes its results where the backward one reads its inputs
+        sweep_f.fill(SW_DIV, Lrp.get(), Lci.get(), Lv.get(), SD_LAST, nullptr, sweep_b.pos.get(), lo, s);
+        sweep_b.fill(SW_ICB, Urp.get(), Uci.get(), Uv.get(), SD_ARRAY, inv.get(), nullptr, lo, s);
+        return nk + 2;
+    }
     if (lo) {
         nk += 3;
         Lv_lo.alloc(nl); Uv_lo.alloc(nu); inv_lo.alloc(n);
@@ -625,6 +633,11 @@ template <typename S>
 void ICDevice<S>::apply_fwd(const S* x, const KState* st, cudaStream_t s) const {
     const int* uo = abmc ? uoff.get() : nullptr;
     const double* sc = scaled_apply ? scaling.get() : nullptr;
+    if (swept()) {
+        sweep_f.load(x, nullptr, sc, st, s);
+        sweep_f.run(sweep_b.xs.get(), st, s);
+        return;
+    }
     if (blk) {
         if (lo) {
             SSV_BLK_DISPATCH(launch_fwd_blk, SL, *this, ev_lo.get(), iv_lo.get(), dv_lo.get(), x, sc, st, s)
@@ -651,6 +664,12 @@ template <typename S>
 void ICDevice<S>::apply_bwd(S* y, const KState* st, cudaStream_t s) const {
     const int* uo = abmc ? uoff.get() : nullptr;
     const double* sc = scaled_apply ? scaling.get() : nullptr;
+    if (swept()) {
+        sweep_b.run(y, st, s);
+        if (sc) launch_k(k_scale_real<S>, grid_for(n, kBlock), kBlock, s, n, y, sc);
+        SSV_LAUNCH_CHECK();
+        return;
+    }
     if (blk) {
         if (lo) {
             SSV_BLK_DISPATCH(launch_bwd_blk, SL, *this, uev_lo.get(), iv_lo.get(), inv_lo.get(), y, st, s)
@@ -822,7 +841,7 @@ static void run_krylov(ssv_solver* sv, int method, const ssv_config& cfg, const 
     std::string key;
     if (method == SSV_METHOD_CG || method == SSV_METHOD_ICCG) {
         // z = M^{-1} r, rho = (r, z), p = z (cg_solver.hpp:428-432)
-        if (ic) ic->apply(w.r.get(), w.z.get(), nullptr, s);
+        if (ic) ic->apply(w.r.get(), w.z.get(), cfg.max_iterations > 0 ? dst : nullptr, s);
         launch_k(k_dot<S>, g, kBlock, s, n, w.r.get(), z, cfg.conjugate, nullptr, RED_STORE, red, &dst->rho);
         launch_k(k_copy<S>, g, kBlock, s, n, z, w.p.get());
         SSV_LAUNCH_CHECK();
@@ -830,7 +849,8 @@ static void run_krylov(ssv_solver* sv, int method, const ssv_config& cfg, const 
         key = "cg" + std::to_string(method) + ";" + std::to_string(n) + ";" + std::to_string(lanes) + ";" +
               ptr_key(wrp) + ptr_key(wv) + ptr_key(w.r.get()) + ptr_key(dst) +
               ptr_key(red.partials) + std::to_string(fd != nullptr) +
-              (ic ? ptr_key(ic) + std::to_string(ic->gen) + ";" + ptr_key(ic->Lv.get()) + ptr_key(ic->Lv_lo.get()) + std::to_string(ic->lo) +
+              (ic ? ptr_key(ic) + std::to_string(ic->gen) + ";" + ptr_key(ic->Lv.get()) + ptr_key(ic->Lv_lo.get()) + ptr_key(ic->sweep_f.stream.get()) +
+                        ptr_key(ic->sweep_b.stream.get()) + std::to_string(ic->lo) +
                         std::to_string(ic->scaled_apply) + std::to_string(ic->fwd_launch.size())
                   : std::string());
         build_graph_loop(sv->loop, key, [&](cudaGraphConditionalHandle hc, int use_cond) {
@@ -999,8 +1019,8 @@ static void profile_krylov(ssv_solver* sv, int method, const ssv_config& cfg, in
         if (ic) {
             const double ZL = (double)ic->h_Lci.size();
             const double lb = ic->lo ? sizeof(typename ST<S>::lo) : sb;
-            const int kf = ic->blk ? (int)ic->fwd_cta.size() : (int)ic->fwd_launch.size();
-            const int kb = ic->blk ? (int)ic->bwd_cta.size() : (int)ic->bwd_launch.size();
+            const int kf = ic->swept() ? 2 : ic->blk ? (int)ic->fwd_cta.size() : (int)ic->fwd_launch.size();
+            const int kb = ic->swept() ? 1 : ic->blk ? (int)ic->bwd_cta.size() : (int)ic->bwd_launch.size();
             timed("ic_forward", ZL * (4 + lb) + (N + 1) * 4 + 2 * N * sb, kf,
                   [&] { ic->apply_fwd(w.r.get(), dst, s); });
             timed("ic_backward", ZL * (4 + lb) + (N + 1) * 4 + N * lb + 2 * N * sb,
@@ -1118,6 +1138,23 @@ void precond_apply_dev(ssv_precond* p, const void* d_x, void* d_y) {
         precond_apply_any<zdouble>(p, static_cast<const zdouble*>(d_x), static_cast<zdouble*>(d_y), nullptr,
                                    stream());
     SSV_CUDA(cudaStreamSynchronize(stream()));
+    precond_check(p, stream());
+}
+
+void precond_check(const ssv_precond* p, cudaStream_t s) {
+    auto sweeps = [&](auto& q) {
+        if (q.swept()) {
+            q.sweep_f.check(s);
+            q.sweep_b.check(s);
+        }
+    };
+    if (p && p->kind == 1) {
+        if (p->A->dtype == SSV_F64) sweeps(p->ic_d);
+        else sweeps(p->ic_z);
+    } else if (p && p->kind == 4) {
+        if (p->A->dtype == SSV_F64) sweeps(p->sgs_d);
+        else sweeps(p->sgs_z);
+    }
 }
 
 double precond_actual_shift(const ssv_precond* p) {

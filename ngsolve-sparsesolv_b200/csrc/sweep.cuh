@@ -1,0 +1,76 @@
+// sweep.cuh -- level-scheduled triangular sweeps in one launch.
+//
+// A sweep y_i = f(x_i, sum over j before i of a_ij y_j) is a chain of level
+// sets: 100 to 600 of them on nodal and edge-element matrices, a few hundred to
+// a few thousand rows each. One launch per level costs 2.4 - 3.0 us a level
+// whatever the level holds. Here one thread-block cluster (2 - 16 CTAs, by the
+// mean level width) walks all levels:
+//   - every CTA owns a part of each level; its rows' records (coefficients,
+//     columns, diagonal, output index) are one contiguous stream, and a
+//     producer warp moves it and the inputs, which lie in the same order, into
+//     a ring of shared-memory stages with bulk copies, ahead of the chain; four
+//     groups of four warps take the rounds in turn;
+//   - a row's result goes to the shared-memory windows of exactly those CTAs
+//     that need it, by st.async, which also counts the bytes into the level's
+//     mbarrier there: no barrier over the cluster and no fence on the chain;
+//   - where the windows cannot hold all results, the levels form chunks; between
+//     chunks the cluster meets once, and couplings to earlier chunks are read
+//     from the output in memory.
+// A record holds the row's coefficients already scaled by its diagonal, so that
+// y_i = scale_i x_i - sum a'_ij y_j has no division and no multiplication after
+// the sum. Entries of levels before the last one ("early") are summed before the
+// last level's results are waited for.
+#pragma once
+
+#include "ssv_common.cuh"
+#include "sweep_plan.hpp"
+
+namespace ssv {
+
+struct KState;
+
+// What a sweep computes, with d the row's diagonal value of fill():
+enum SweepOp : int {
+    SW_DIV = 0,  // y = (x - sum) / d
+    SW_MUL,      // y = (x - sum) * d
+    SW_ICB,      // y = x - sum * d (also (x / d - sum) * d)
+};
+
+// where a row's d comes from
+enum SweepDiag : int { SD_LAST = 0, SD_FIRST = 1, SD_ARRAY = 2 };
+
+template <typename S>
+struct Sweep {
+    SweepPlanHost plan;
+    bool ready = false;
+    bool fwd = true;
+    int stages = 0, smem = 0;
+    bool lo = false;
+    DevBuf<unsigned char> stream;
+    DevBuf<int> rowpos, pos, lev, tgt_ptr, tgt, slice_round, slice_chunk0, slice_off16, round_ptr, chunk_lev, err;
+    DevBuf<uint8_t> cta;
+    DevBuf<uint32_t> tx;
+    DevBuf<SweepRound> rounds;
+    DevBuf<S> xs;  // inputs by position
+
+    // Plans the sweep for a triangular part of the pattern (entries j < i or
+    // j > i of every row); false (and ready = false) where it does not fit --
+    // the caller then launches level by level.
+    bool build(int n, const std::vector<int>& rp, const std::vector<int>& ci, bool fwd,
+               const std::vector<int>& rows, const std::vector<int>& off, cudaStream_t s);
+    // Writes the records from the CSR values: d from the row's last or first
+    // entry or from darr; omap = output index of every row (null = the row).
+    // lo_ stores the coefficients in the FP32 form.
+    void fill(SweepOp op, const int* rp, const int* ci, const S* v, int dmode, const S* darr, const int* omap,
+              bool lo_, cudaStream_t s);
+    // xs[position] = sc * a - b of its row (sc, b may be null)
+    void load(const S* a, const S* b, const double* sc, const KState* st, cudaStream_t s) const;
+    // Sweeps from xs into out (at the rows' output indices).
+    void run(S* out, const KState* st, cudaStream_t s) const;
+    // After the stream has been waited for: raises SSV_ERR_TIMEOUT if a bounded
+    // wait of a sweep outside a solve's state gave up.
+    void check(cudaStream_t s) const;
+    int positions() const { return plan.nslices * 32; }
+};
+
+}  // namespace ssv

@@ -616,103 +616,12 @@ k_ic_bwd(int u0, int u1, const int* __restrict__ uoff, const int* __restrict__ r
     }
 }
 
-// ---------------------------------------------------------------------------
-// ABMC block sweeps, one sub-warp of LANES (>= rows per block) lanes per
-// ABMC block: lane j owns row r0+j. The terms coupling a row to rows of
-// earlier colours ("external", a CSR without the block's own columns) are
-// gathered by all lanes at once; the couplings inside the block come from a
-// packed strictly-lower table (entry (j,t) at j*(j-1)/2+t) and are resolved
-// row by row through register shuffles. The loops are warp-uniform.
-// ---------------------------------------------------------------------------
 template <typename S>
 __device__ __forceinline__ S shfl_s(S v, int src, int width) {
     if constexpr (ST<S>::cplx) {
         return S{__shfl_sync(0xffffffffu, v.x, src, width), __shfl_sync(0xffffffffu, v.y, src, width)};
     } else {
         return __shfl_sync(0xffffffffu, v, src, width);
-    }
-}
-
-// forward: y_i = (x_i*sc_i - sum_ext L_ik y_k - sum_{t<j} L_jt y_t) / L_ii
-template <typename S, typename SL, int LANES>
-__global__ void __launch_bounds__(128)
-k_ic_fwd_blk(int b0, int b1, const int* __restrict__ boff, const int* __restrict__ erp,
-             const int* __restrict__ eci, const SL* __restrict__ ev, const SL* __restrict__ iv, int tri,
-             const SL* __restrict__ dv, const S* __restrict__ x, const double* __restrict__ sc,
-             S* __restrict__ y, const KState* st) {
-    pdl_gate();
-    if (st && st->done) return;
-    const int lane = threadIdx.x % LANES;
-    const int gw = (threadIdx.x & 31) / LANES;
-    const int stride = gridDim.x * (blockDim.x / LANES);
-    for (int b = b0 + blockIdx.x * (blockDim.x / LANES) + threadIdx.x / LANES; b - gw < b1; b += stride) {
-        const bool vb = b < b1;
-        int r0 = 0, nr = 0;
-        if (vb) { r0 = boff[b]; nr = boff[b + 1] - r0; }
-        const bool act = vb && lane < nr;
-        const int i = r0 + lane;
-        S s = ST<S>::zero();
-        if (act) {
-            s = x[i];
-            if (sc) s = ST<S>::scale(sc[i], s);
-            const int k1 = erp[i + 1];
-            for (int k = erp[i]; k < k1; ++k) s = s - hi_of_any(ev[k]) * y[eci[k]];
-        }
-        S yi = ST<S>::zero();
-        const SL* ib = iv + (size_t)(vb ? b : 0) * tri;
-#pragma unroll
-        for (int t = 0; t < LANES; ++t) {
-            if (act && lane == t) yi = ST<S>::div(s, hi_of_any(dv[i]));
-            const S yt = shfl_s(yi, t, LANES);
-            if (act && t < lane) s = s - hi_of_any(ib[lane * (lane - 1) / 2 + t]) * yt;
-        }
-        if (act) y[i] = yi;
-    }
-}
-
-// backward: y_i = -(sum_ext U_ik y_k + sum_{t>j} L_tj y_t) * D^{-1}_i + x_i
-template <typename S, typename SL, int LANES>
-__global__ void __launch_bounds__(128)
-k_ic_bwd_blk(int b0, int b1, const int* __restrict__ boff, const int* __restrict__ urp,
-             const int* __restrict__ uci, const SL* __restrict__ uv, const SL* __restrict__ iv, int tri,
-             const SL* __restrict__ inv, const S* __restrict__ x, S* __restrict__ y, const KState* st) {
-    pdl_gate();
-    if (st && st->done) return;
-    const int lane = threadIdx.x % LANES;
-    const int gw = (threadIdx.x & 31) / LANES;
-    const int stride = gridDim.x * (blockDim.x / LANES);
-    for (int b = b0 + blockIdx.x * (blockDim.x / LANES) + threadIdx.x / LANES; b - gw < b1; b += stride) {
-        const bool vb = b < b1;
-        int r0 = 0, nr = 0;
-        if (vb) { r0 = boff[b]; nr = boff[b + 1] - r0; }
-        const bool act = vb && lane < nr;
-        const int i = r0 + lane;
-        S s = ST<S>::zero();
-        if (act) {
-            const int k1 = urp[i + 1];
-            for (int k = urp[i]; k < k1; ++k) s = s - hi_of_any(uv[k]) * y[uci[k]];
-        }
-        S yi = ST<S>::zero();
-        const SL* ib = iv + (size_t)(vb ? b : 0) * tri;
-#pragma unroll
-        for (int t = LANES - 1; t >= 0; --t) {
-            if (act && lane == t) yi = s * hi_of_any(inv[i]) + x[i];
-            const S yt = shfl_s(yi, t, LANES);
-            if (act && lane < t && t < nr) s = s - hi_of_any(ib[t * (t - 1) / 2 + lane]) * yt;
-        }
-        if (act) y[i] = yi;
-    }
-}
-
-// out[k] = src[map[k]], or zero where map[k] < 0
-template <typename S, typename SO>
-__global__ void k_gather_or_zero(int64_t m, const int* __restrict__ map, const S* __restrict__ src,
-                                 SO* __restrict__ out) {
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < m;
-         k += (int64_t)gridDim.x * blockDim.x) {
-        const int q = map[k];
-        if constexpr (std::is_same<S, SO>::value) out[k] = q >= 0 ? src[q] : ST<S>::zero();
-        else out[k] = lo_of(q >= 0 ? src[q] : ST<S>::zero());
     }
 }
 
@@ -763,110 +672,12 @@ k_ic_bwd_cta(int nlev, const int* __restrict__ lev, const int* __restrict__ rows
     }
 }
 
-// Oversized ABMC block, staged: the block's rows, their L (forward) or U
-// (backward) entries and the values of the couplings to other blocks (final
-// before the launch) are copied into shared memory first, so the chain of
-// level sets touches only shared memory. Same per-row arithmetic, in the same
-// order, as k_ic_fwd_cta / k_ic_bwd_cta. Per-row entry lists: srp (by position
-// in rows[]), value index ssrc, column scol, and sloc = the column's position
-// within the block (relative to lev[0]) or -1 for a coupling outside it.
-template <typename S, typename SL>
-struct StagedSmem {
-    S* ys;
-    S* xs;
-    S* eext;
-    SL* dg;
-    SL* ev;
-    int* eloc;
-    int* slev;
-    int* srow;
-};
-
-__host__ __device__ inline size_t staged_align(size_t b) { return (b + 15) & ~size_t(15); }
-
-template <typename S, typename SL>
-__host__ __device__ inline size_t staged_bytes(int nr, int ne, int nlev) {
-    return 2 * staged_align((size_t)nr * sizeof(S)) + staged_align((size_t)ne * sizeof(S)) +
-           staged_align((size_t)nr * sizeof(SL)) + staged_align((size_t)ne * sizeof(SL)) +
-           staged_align((size_t)ne * 4) + staged_align((size_t)(nlev + 1) * 4) + staged_align((size_t)(nr + 1) * 4);
-}
-
 // Loads of values that other CTAs of the same launch may have written: served
 // by L2 (the point of coherence), never by a possibly stale L1 line.
 __device__ __forceinline__ double ld_cg(const double* p) { return __ldcg(p); }
 __device__ __forceinline__ zdouble ld_cg(const zdouble* p) {
     const double2 v = __ldcg(reinterpret_cast<const double2*>(p));
     return {v.x, v.y};
-}
-
-template <typename S, typename SL, bool FWD>
-__device__ __forceinline__ void staged_sweep(unsigned char* smem, int nlev, const int* __restrict__ lev,
-                                             const int* __restrict__ rows, const int* __restrict__ srp,
-                                             const int* __restrict__ ssrc, const int* __restrict__ scol,
-                                             const int* __restrict__ sloc, const int* __restrict__ Lrp,
-                                             const SL* __restrict__ vals, const SL* __restrict__ inv_diag,
-                                             const S* __restrict__ x, const double* __restrict__ sc, S* y) {
-    const int qa = lev[0], qb = lev[nlev];
-    const int nr = qb - qa;
-    const int ea = srp[qa], ne = srp[qb] - ea;
-    unsigned char* p = smem;
-    S* ys = reinterpret_cast<S*>(p);   p += staged_align((size_t)nr * sizeof(S));
-    S* xs = reinterpret_cast<S*>(p);   p += staged_align((size_t)nr * sizeof(S));
-    S* eext = reinterpret_cast<S*>(p); p += staged_align((size_t)ne * sizeof(S));
-    SL* dg = reinterpret_cast<SL*>(p); p += staged_align((size_t)nr * sizeof(SL));
-    SL* ev = reinterpret_cast<SL*>(p); p += staged_align((size_t)ne * sizeof(SL));
-    int* eloc = reinterpret_cast<int*>(p); p += staged_align((size_t)ne * 4);
-    int* slev = reinterpret_cast<int*>(p); p += staged_align((size_t)(nlev + 1) * 4);
-    int* srow = reinterpret_cast<int*>(p);
-    for (int l = threadIdx.x; l <= nlev; l += blockDim.x) slev[l] = lev[l] - qa;
-    for (int q = threadIdx.x; q <= nr; q += blockDim.x) srow[q] = srp[qa + q] - ea;
-    for (int q = threadIdx.x; q < nr; q += blockDim.x) {
-        const int i = rows[qa + q];
-        if constexpr (FWD) {
-            S v = x[i];
-            if (sc) v = ST<S>::scale(sc[i], v);
-            xs[q] = v;
-            dg[q] = vals[Lrp[i + 1] - 1];
-        } else {
-            xs[q] = x[i];
-            dg[q] = inv_diag[i];
-        }
-    }
-    for (int e = threadIdx.x; e < ne; e += blockDim.x) {
-        const int loc = sloc[ea + e];
-        eloc[e] = loc;
-        ev[e] = vals[ssrc[ea + e]];
-        eext[e] = loc < 0 ? ld_cg(y + scol[ea + e]) : ST<S>::zero();
-    }
-    __syncthreads();
-    for (int l = 0; l < nlev; ++l) {
-        const int q1 = slev[l + 1];
-        for (int q = slev[l] + threadIdx.x; q < q1; q += blockDim.x) {
-            S s = FWD ? xs[q] : ST<S>::zero();
-            const int e1 = srow[q + 1];
-            for (int e = srow[q]; e < e1; ++e) {
-                const int loc = eloc[e];
-                const S yv = loc < 0 ? eext[e] : ys[loc];
-                s = s - hi_of_any(ev[e]) * yv;
-            }
-            if constexpr (FWD) ys[q] = ST<S>::div(s, hi_of_any(dg[q]));
-            else ys[q] = s * hi_of_any(dg[q]) + xs[q];
-        }
-        __syncthreads();
-    }
-    for (int q = threadIdx.x; q < nr; q += blockDim.x) y[rows[qa + q]] = ys[q];
-}
-
-template <typename S, typename SL, bool FWD>
-__global__ void __launch_bounds__(256)
-k_ic_sweep_staged(int nlev, const int* __restrict__ lev, const int* __restrict__ rows, const int* __restrict__ srp,
-                  const int* __restrict__ ssrc, const int* __restrict__ scol, const int* __restrict__ sloc,
-                  const int* __restrict__ Lrp, const SL* __restrict__ vals, const SL* __restrict__ inv_diag,
-                  const S* __restrict__ x, const double* __restrict__ sc, S* y, const KState* st) {
-    pdl_gate();
-    if (st && st->done) return;
-    extern __shared__ __align__(16) unsigned char smem[];
-    staged_sweep<S, SL, FWD>(smem, nlev, lev, rows, srp, ssrc, scol, sloc, Lrp, vals, inv_diag, x, sc, y);
 }
 
 }  // namespace ssv

@@ -8,6 +8,7 @@
 
 #include "host_order.hpp"
 #include "kernels.cuh"
+#include "block_sweep.cuh"
 #include "sell.cuh"
 #include "sweep.cuh"
 
@@ -229,27 +230,17 @@ struct ICDevice {
     int missing_row = -1;
     double actual_shift = 0.0;
     DevBuf<S> tw;  // forward-sweep output
-    // level schedule: both sweeps in one launch each (else level by level)
+    // both sweeps in one launch each (sweep.cuh); else level by level, or (ABMC) colour by colour
     Sweep<S> sweep_f, sweep_b;
-    bool swept() const { return !abmc && missing_row < 0 && sweep_f.ready && sweep_b.ready; }
-    // ABMC block-sweep layout (k_ic_fwd_blk / k_ic_bwd_blk): external parts of
-    // L and U rows, packed strictly-lower intra-block table, diagonal
+    bool swept() const { return missing_row < 0 && sweep_f.ready && sweep_b.ready; }
+    // ABMC: colour by colour in the block layout (block_sweep.cuh), or by the
+    // CSR factor where a block is too large for that
     bool blk = false;
-    int blk_lanes = 0, tri = 1;
-    // launches of the block sweeps in processing order: kind 0 = range of
-    // ordinary blocks [a, b) (sub-warp kernels), kind 1 = range [a, b) of the
-    // rows_f / rows_b lists (one level of an oversized block; factorisation),
-    // kind 2 = an oversized block swept by one CTA over the level offsets
-    // lev_f / lev_b [a, b] (apply)
-    struct Launch { int kind, a, b, smem = 0, color = -1; };  // smem > 0: oversized block swept staged (bytes)
-    std::vector<Launch> fwd_blk, bwd_blk, fwd_cta, bwd_cta;
-    DevBuf<int> lev_f, lev_b;
-    // staged sweeps of oversized blocks: per position in rows_f / rows_b, the
-    // row's entries (value index, column, position in the block or -1)
-    DevBuf<int> sf_rp, sf_src, sf_col, sf_loc, sb_rp, sb_src, sb_col, sb_loc;
-    DevBuf<int> erp, eci, esrc, urpe, ucie, usrce, isrc, dsrc;
-    DevBuf<S> ev, uev, iv, dv;
-    DevBuf<SL> ev_lo, uev_lo, iv_lo, dv_lo;
+    BlockSweep<S> blocks;
+    // launches of the ABMC factorisation: kind 0 = range of ordinary blocks [a, b),
+    // kind 1 = range [a, b) of rows_f (one level of an oversized block)
+    struct Launch { int kind, a, b; };
+    std::vector<Launch> fwd_blk;
 
     // Pattern set-up from the matrix pattern (host) for the given options.
     void build_pattern(int n, const std::vector<int>& rp, const std::vector<int>& ci,
@@ -268,8 +259,7 @@ struct ICDevice {
     int kernels_per_apply() const {
         if (swept()) return 3 + (scaled_apply ? 1 : 0);
         if (blk)
-            return (int)fwd_cta.size() + (int)bwd_cta.size() +
-                   (scaled_apply ? 1 : 0);
+            return (int)(blocks.f.steps.size() + blocks.b.steps.size()) + (scaled_apply ? 1 : 0);
         return (int)(fwd_launch.size() + bwd_launch.size()) + (scaled_apply ? 1 : 0);
     }
 };

@@ -180,6 +180,7 @@ void ICDevice<S>::build_pattern(int n_, const std::vector<int>& rp, const std::v
     nct = cfg.abmc_num_colors;
     fwd_launch.clear();
     bwd_launch.clear();
+    sweep_f.ready = sweep_b.ready = false;
     std::vector<int> lrp, lci, lsrc, urp, uci, usrc;
     if (abmc) {
         // abmc_use_rcm (ic_preconditioner.hpp:97-104): the ABMC schedule is
@@ -265,9 +266,6 @@ void ICDevice<S>::build_pattern(int n_, const std::vector<int>& rp, const std::v
     if (!flag.get()) flag.alloc(1);
     blk = false;
     fwd_blk.clear();
-    bwd_blk.clear();
-    fwd_cta.clear();
-    bwd_cta.clear();
     if (abmc && missing_row < 0 && cfg.abmc_block_size <= 32) {
         // Ordinary blocks hold <= block_size rows; the aggregation appends any
         // rows it could not place to the last block
@@ -281,42 +279,12 @@ void ICDevice<S>::build_pattern(int n_, const std::vector<int>& rp, const std::v
             if (sz <= cap) bsmax = std::max(bsmax, sz);
         }
         blk = true;
-        blk_lanes = 1;
-        while (blk_lanes < bsmax) blk_lanes <<= 1;
-        tri = std::max(1, bsmax * (bsmax - 1) / 2);
-        std::vector<int> h_erp(n + 1, 0), h_eci, h_esrc, h_urp(n + 1, 0), h_uci, h_usrc, h_dsrc(n);
-        std::vector<int> h_isrc((size_t)num_blocks * tri, -1);
-        std::vector<int> h_rows_f, h_rows_b, h_lev_f, h_lev_b;
-        std::vector<int> h_sf_rp(1, 0), h_sf_src, h_sf_col, h_sf_loc, h_sb_rp(1, 0), h_sb_src, h_sb_col, h_sb_loc;
-        std::vector<int> pos;
-        int smem_optin = 0, staged_max = 0;
-        SSV_CUDA(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, 0));
-        h_eci.reserve(lci.size());
-        h_esrc.reserve(lci.size());
-        h_uci.reserve(uci.size());
-        h_usrc.reserve(uci.size());
-        std::vector<int> lev;
-        for (int b = 0; b < num_blocks; ++b) {
-            const int r0 = bo[b], r1 = bo[b + 1];
-            const bool big = (r1 - r0) > cap;
-            for (int i = r0; i < r1; ++i) {
-                for (int k = lrp[i]; k < lrp[i + 1] - 1; ++k) {
-                    const int c = lci[k];
-                    if (c < r0 || big) { h_eci.push_back(c); h_esrc.push_back(k); }
-                    else {
-                        const int j = i - r0, t = c - r0;
-                        h_isrc[(size_t)b * tri + j * (j - 1) / 2 + t] = k;
-                    }
-                }
-                h_erp[i + 1] = (int)h_eci.size();
-                h_dsrc[i] = lrp[i + 1] - 1;
-                for (int k = urp[i] + 1; k < urp[i + 1]; ++k)
-                    if (uci[k] >= r1 || big) { h_uci.push_back(uci[k]); h_usrc.push_back(usrc[k]); }
-                h_urp[i + 1] = (int)h_uci.size();
-            }
-        }
-        // launch lists: colour by colour; runs of ordinary blocks, and the
-        // level sets of oversized blocks (forward: dependencies on earlier
+        int lanes_blk = 1;
+        while (lanes_blk < bsmax) lanes_blk <<= 1;
+        using Run = typename BlockSweep<S>::Run;
+        std::vector<Run> run_f, run_b;
+        std::vector<int> h_rows_f, h_rows_b, h_lev_f, h_lev_b, lev;
+        // the level sets of an oversized block (forward: dependencies on earlier
         // rows of the block, backward: on later rows)
         auto add_big = [&](int r0, int r1, bool fwd) {
             const int m = r1 - r0;
@@ -343,89 +311,53 @@ void ICDevice<S>::build_pattern(int n_, const std::vector<int>& rp, const std::v
             std::vector<int>& lv = fwd ? h_lev_f : h_lev_b;
             const int p0 = (int)lv.size();
             lv.push_back((int)rows.size());
-            const int qa = (int)rows.size();
             for (int l = 0; l < nl; ++l) {
                 const int a = (int)rows.size();
                 for (int i = r0; i < r1; ++i)
                     if (lev[i - r0] == l) rows.push_back(i);
-                (fwd ? fwd_blk : bwd_blk).push_back({1, a, (int)rows.size()});
+                if (fwd) fwd_blk.push_back({1, a, (int)rows.size()});
                 lv.push_back((int)rows.size());
             }
-            // staged copy: each row's entries in sweep order, couplings inside
-            // the block by position, the others by column
-            const int qb = (int)rows.size();
-            pos.assign(m, -1);
-            for (int q = qa; q < qb; ++q) pos[rows[q] - r0] = q - qa;
-            std::vector<int>& srp = fwd ? h_sf_rp : h_sb_rp;
-            std::vector<int>& ssrc = fwd ? h_sf_src : h_sb_src;
-            std::vector<int>& scol = fwd ? h_sf_col : h_sb_col;
-            std::vector<int>& sloc = fwd ? h_sf_loc : h_sb_loc;
-            const int e0 = (int)ssrc.size();
-            for (int q = qa; q < qb; ++q) {
-                const int i = rows[q];
-                const int ka = fwd ? lrp[i] : urp[i] + 1, kb = fwd ? lrp[i + 1] - 1 : urp[i + 1];
-                for (int k = ka; k < kb; ++k) {
-                    const int c = fwd ? lci[k] : uci[k];
-                    ssrc.push_back(k);
-                    scol.push_back(c);
-                    sloc.push_back(c >= r0 && c < r1 ? pos[c - r0] : -1);
-                }
-                srp.push_back((int)ssrc.size());
-            }
-            // headroom for the launching kernel's static shared memory
-            const size_t bytes = staged_bytes<S, S>(qb - qa, (int)ssrc.size() - e0, nl);
-            const int smem = bytes + 1024 <= (size_t)smem_optin ? (int)bytes : 0;
-            staged_max = std::max(staged_max, smem);
-            (fwd ? fwd_cta : bwd_cta).push_back({2, p0, p0 + nl, smem});
+            (fwd ? run_f : run_b).push_back({2, p0, p0 + nl});
         };
         auto add_colour = [&](int c, bool fwd) {
             const int b0 = sched_color_offsets[c], b1 = sched_color_offsets[c + 1];
-            std::vector<Launch>& cta = fwd ? fwd_cta : bwd_cta;
             int run = b0;
+            auto blocks_to = [&](int b) {
+                if (b <= run) return;
+                if (fwd) fwd_blk.push_back({0, run, b});
+                (fwd ? run_f : run_b).push_back({0, run, b});
+            };
             for (int b = b0; b < b1; ++b) {
                 if (bo[b + 1] - bo[b] > cap) {
-                    if (b > run) {
-                        (fwd ? fwd_blk : bwd_blk).push_back({0, run, b});
-                        cta.push_back({0, run, b, 0, c});
-                    }
+                    blocks_to(b);
                     add_big(bo[b], bo[b + 1], fwd);
-                    cta.back().color = c;
                     run = b + 1;
                 }
             }
-            if (b1 > run) {
-                (fwd ? fwd_blk : bwd_blk).push_back({0, run, b1});
-                cta.push_back({0, run, b1, 0, c});
-            }
+            blocks_to(b1);
         };
         for (int c = 0; c < num_colors; ++c) add_colour(c, true);
         for (int c = num_colors - 1; c >= 0; --c) add_colour(c, false);
-        erp.upload(h_erp.data(), h_erp.size(), s);
-        eci.upload(h_eci.data(), h_eci.size(), s);
-        esrc.upload(h_esrc.data(), h_esrc.size(), s);
-        urpe.upload(h_urp.data(), h_urp.size(), s);
-        ucie.upload(h_uci.data(), h_uci.size(), s);
-        usrce.upload(h_usrc.data(), h_usrc.size(), s);
-        isrc.upload(h_isrc.data(), h_isrc.size(), s);
-        dsrc.upload(h_dsrc.data(), h_dsrc.size(), s);
-        if (!h_rows_f.empty()) rows_f.upload(h_rows_f.data(), h_rows_f.size(), s);
-        if (!h_rows_b.empty()) rows_b.upload(h_rows_b.data(), h_rows_b.size(), s);
-        if (!h_lev_f.empty()) lev_f.upload(h_lev_f.data(), h_lev_f.size(), s);
-        if (!h_lev_b.empty()) lev_b.upload(h_lev_b.data(), h_lev_b.size(), s);
-        auto up = [&](DevBuf<int>& d, const std::vector<int>& h) {
-            if (!h.empty()) d.upload(h.data(), h.size(), s);
-        };
-        up(sf_rp, h_sf_rp); up(sf_src, h_sf_src); up(sf_col, h_sf_col); up(sf_loc, h_sf_loc);
-        up(sb_rp, h_sb_rp); up(sb_src, h_sb_src); up(sb_col, h_sb_col); up(sb_loc, h_sb_loc);
-        if (staged_max > 0) {  // dynamic shared memory of the staged sweeps (<= optin - 1 KB)
-            using SLo = typename ST<S>::lo;
-            const int sm = staged_max;
-            SSV_CUDA(cudaFuncSetAttribute(k_ic_sweep_staged<S, S, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
-            SSV_CUDA(cudaFuncSetAttribute(k_ic_sweep_staged<S, S, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
-            SSV_CUDA(cudaFuncSetAttribute(k_ic_sweep_staged<S, SLo, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
-            SSV_CUDA(cudaFuncSetAttribute(k_ic_sweep_staged<S, SLo, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+        // Colours of few rows: the factor's own level sets through the one-launch sweeps. A level
+        // takes 0.6 us there while it fills the cluster at most (about 1024 real rows), more in
+        // proportion beyond; a colour's launch takes 2.6 us. Measured forward / backward: 24x25x23
+        // (25 levels of 552 rows, 9 launches) 14.9 / 13.7 against 23.8 / 20.7 us; 64^3 (47 levels
+        // of 5577, 10 launches) 116 / 123 against 38 / 33 us.
+        const int nl = build_levels(n, lrp.data(), lci.data(), false, lev);
+        const double fill = std::max(1.0, (double)n / std::max(nl, 1) * (ST<S>::cplx ? 2 : 1) / 1024.0);
+        if (0.6 * nl * fill < 2.6 * (double)run_f.size()) {
+            std::vector<int> rws, off;
+            group_by_level(lev, nl, rws, off);
+            if (sweep_f.build(n, lrp, lci, true, rws, off, s)) {
+                const int nu = build_levels(n, urp.data(), uci.data(), true, lev);
+                group_by_level(lev, nu, rws, off);
+                sweep_b.build(n, urp, uci, false, rws, off, s);
+            }
         }
-        ev.alloc(h_eci.size()); uev.alloc(h_uci.size()); iv.alloc(h_isrc.size()); dv.alloc(n);
+        if (!swept())
+            blocks.build(lanes_blk, bo, run_f, run_b, h_rows_f, h_lev_f, h_rows_b, h_lev_b, lrp, lci, urp, uci, usrc, s);
+        if (!h_rows_f.empty()) rows_f.upload(h_rows_f.data(), h_rows_f.size(), s);
     }
     built = true;
     SSV_CUDA(cudaStreamSynchronize(s));
@@ -530,20 +462,6 @@ int ICDevice<S>::factorize(const S* vals, const ssv_config& cfg) {
     SSV_LAUNCH_CHECK();
     ++nk;
     lo = cfg.precision == SSV_PREC_FP32;
-    if (blk) {
-        auto gz = [&](const DevBuf<int>& src, auto& out) {
-            const int64_t m = (int64_t)src.size();
-            if (m > 0) k_gather_or_zero<S><<<grid_for(m, kBlock), kBlock, 0, s>>>(m, src.get(), Lv.get(), out.get());
-            ++nk;
-        };
-        if (lo) {
-            ev_lo.alloc(ev.size()); uev_lo.alloc(uev.size()); iv_lo.alloc(iv.size()); dv_lo.alloc(n);
-            gz(esrc, ev_lo); gz(usrce, uev_lo); gz(isrc, iv_lo); gz(dsrc, dv_lo);
-        } else {
-            gz(esrc, ev); gz(usrce, uev); gz(isrc, iv); gz(dsrc, dv);
-        }
-        SSV_LAUNCH_CHECK();
-    }
     if (swept()) {
         // the forward sweep writes its results where the backward one reads its inputs
         sweep_f.fill(SW_DIV, Lrp.get(), Lci.get(), Lv.get(), SD_LAST, nullptr, sweep_b.pos.get(), lo, s);
@@ -558,76 +476,15 @@ int ICDevice<S>::factorize(const S* vals, const ssv_config& cfg) {
         k_to_lo<S, SL><<<grid_for(n, kBlock), kBlock, 0, s>>>(n, inv.get(), inv_lo.get());
         SSV_LAUNCH_CHECK();
     }
+    if (blk) {
+        blocks.Lrp = Lrp.get(); blocks.Lci = Lci.get(); blocks.Lv = Lv.get(); blocks.Lv_lo = Lv_lo.get();
+        blocks.Urp = Urp.get(); blocks.Uci = Uci.get(); blocks.Uv = Uv.get(); blocks.Uv_lo = Uv_lo.get();
+        blocks.inv = inv.get(); blocks.inv_lo = inv_lo.get();
+        blocks.fill(lo, s);
+        nk += 2;
+    }
     return nk;
 }
-
-// one CTA of 256 threads with `smem` bytes of dynamic shared memory, PDL allowed
-template <typename... KArgs, typename... Args>
-static void launch_staged(void (*k)(KArgs...), int smem, cudaStream_t s, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(1);
-    cfg.blockDim = dim3(256);
-    cfg.dynamicSmemBytes = (size_t)smem;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = pdl_enabled() ? 1 : 0;
-    SSV_CUDA(cudaLaunchKernelEx(&cfg, k, static_cast<KArgs>(args)...));
-}
-
-template <typename S, typename SL, int L>
-static void launch_fwd_blk(const ICDevice<S>& ic, const SL* ev, const SL* iv, const SL* dv, const S* x,
-                           const double* sc, const KState* st, cudaStream_t s) {
-    constexpr int per_cta = 128 / L;
-    const SL* Lfull = ic.lo ? reinterpret_cast<const SL*>(ic.Lv_lo.get()) : reinterpret_cast<const SL*>(ic.Lv.get());
-    for (const auto& g : ic.fwd_cta) {
-        const int units = g.b - g.a;
-        if (units <= 0) continue;
-        if (g.kind == 0)
-            launch_k(k_ic_fwd_blk<S, SL, L>, (units + per_cta - 1) / per_cta, 128, s, 
-                g.a, g.b, ic.uoff.get(), ic.erp.get(), ic.eci.get(), ev, iv, ic.tri, dv, x, sc, ic.tw.get(), st);
-        else if (g.smem > 0)
-            launch_staged(k_ic_sweep_staged<S, SL, true>, g.smem, s, units, ic.lev_f.get() + g.a, ic.rows_f.get(),
-                          ic.sf_rp.get(), ic.sf_src.get(), ic.sf_col.get(), ic.sf_loc.get(), ic.Lrp.get(), Lfull,
-                          (const SL*)nullptr, x, sc, ic.tw.get(), st);
-        else
-            launch_k(k_ic_fwd_cta<S, SL>, 1, 256, s, units, ic.lev_f.get() + g.a, ic.rows_f.get(), ic.Lrp.get(),
-                                                  ic.Lci.get(), Lfull, x, sc, ic.tw.get(), st);
-    }
-}
-
-template <typename S, typename SL, int L>
-static void launch_bwd_blk(const ICDevice<S>& ic, const SL* uev, const SL* iv, const SL* inv, S* y,
-                           const KState* st, cudaStream_t s) {
-    constexpr int per_cta = 128 / L;
-    const SL* Ufull = ic.lo ? reinterpret_cast<const SL*>(ic.Uv_lo.get()) : reinterpret_cast<const SL*>(ic.Uv.get());
-    for (const auto& g : ic.bwd_cta) {
-        const int units = g.b - g.a;
-        if (units <= 0) continue;
-        if (g.kind == 0)
-            launch_k(k_ic_bwd_blk<S, SL, L>, (units + per_cta - 1) / per_cta, 128, s, 
-                g.a, g.b, ic.uoff.get(), ic.urpe.get(), ic.ucie.get(), uev, iv, ic.tri, inv, ic.tw.get(), y, st);
-        else if (g.smem > 0)
-            launch_staged(k_ic_sweep_staged<S, SL, false>, g.smem, s, units, ic.lev_b.get() + g.a, ic.rows_b.get(),
-                          ic.sb_rp.get(), ic.sb_src.get(), ic.sb_col.get(), ic.sb_loc.get(), (const int*)nullptr,
-                          Ufull, inv, (const S*)ic.tw.get(), (const double*)nullptr, y, st);
-        else
-            launch_k(k_ic_bwd_cta<S, SL>, 1, 256, s, units, ic.lev_b.get() + g.a, ic.rows_b.get(), ic.Urp.get(),
-                                                  ic.Uci.get(), Ufull, inv, ic.tw.get(), y, st);
-    }
-}
-
-#define SSV_BLK_DISPATCH(FN, SLT, ...)                         \
-    switch (blk_lanes) {                                      \
-        case 1: FN<S, SLT, 1>(__VA_ARGS__); break;            \
-        case 2: FN<S, SLT, 2>(__VA_ARGS__); break;            \
-        case 4: FN<S, SLT, 4>(__VA_ARGS__); break;            \
-        case 8: FN<S, SLT, 8>(__VA_ARGS__); break;            \
-        case 16: FN<S, SLT, 16>(__VA_ARGS__); break;          \
-        default: FN<S, SLT, 32>(__VA_ARGS__); break;          \
-    }
 
 template <typename S>
 void ICDevice<S>::apply_fwd(const S* x, const KState* st, cudaStream_t s) const {
@@ -639,12 +496,7 @@ void ICDevice<S>::apply_fwd(const S* x, const KState* st, cudaStream_t s) const 
         return;
     }
     if (blk) {
-        if (lo) {
-            SSV_BLK_DISPATCH(launch_fwd_blk, SL, *this, ev_lo.get(), iv_lo.get(), dv_lo.get(), x, sc, st, s)
-        } else {
-            SSV_BLK_DISPATCH(launch_fwd_blk, S, *this, ev.get(), iv.get(), dv.get(), x, sc, st, s)
-        }
-        SSV_LAUNCH_CHECK();
+        blocks.forward(x, sc, tw.get(), st, s);
         return;
     }
     for (const auto& g : fwd_launch) {
@@ -671,11 +523,7 @@ void ICDevice<S>::apply_bwd(S* y, const KState* st, cudaStream_t s) const {
         return;
     }
     if (blk) {
-        if (lo) {
-            SSV_BLK_DISPATCH(launch_bwd_blk, SL, *this, uev_lo.get(), iv_lo.get(), inv_lo.get(), y, st, s)
-        } else {
-            SSV_BLK_DISPATCH(launch_bwd_blk, S, *this, uev.get(), iv.get(), inv.get(), y, st, s)
-        }
+        blocks.backward(tw.get(), y, st, s);
         if (sc) launch_k(k_scale_real<S>, grid_for(n, kBlock), kBlock, s, n, y, sc);
         SSV_LAUNCH_CHECK();
         return;
@@ -850,7 +698,8 @@ static void run_krylov(ssv_solver* sv, int method, const ssv_config& cfg, const 
               ptr_key(wrp) + ptr_key(wv) + ptr_key(w.r.get()) + ptr_key(dst) +
               ptr_key(red.partials) + std::to_string(fd != nullptr) +
               (ic ? ptr_key(ic) + std::to_string(ic->gen) + ";" + ptr_key(ic->Lv.get()) + ptr_key(ic->Lv_lo.get()) + ptr_key(ic->sweep_f.stream.get()) +
-                        ptr_key(ic->sweep_b.stream.get()) + std::to_string(ic->lo) +
+                        ptr_key(ic->sweep_b.stream.get()) + ptr_key(ic->blocks.f.v.get()) + ptr_key(ic->blocks.f.v_lo.get()) +
+                        std::to_string(ic->lo) +
                         std::to_string(ic->scaled_apply) + std::to_string(ic->fwd_launch.size())
                   : std::string());
         build_graph_loop(sv->loop, key, [&](cudaGraphConditionalHandle hc, int use_cond) {
@@ -1019,8 +868,8 @@ static void profile_krylov(ssv_solver* sv, int method, const ssv_config& cfg, in
         if (ic) {
             const double ZL = (double)ic->h_Lci.size();
             const double lb = ic->lo ? sizeof(typename ST<S>::lo) : sb;
-            const int kf = ic->swept() ? 2 : ic->blk ? (int)ic->fwd_cta.size() : (int)ic->fwd_launch.size();
-            const int kb = ic->swept() ? 1 : ic->blk ? (int)ic->bwd_cta.size() : (int)ic->bwd_launch.size();
+            const int kf = ic->swept() ? 2 : ic->blk ? (int)ic->blocks.f.steps.size() : (int)ic->fwd_launch.size();
+            const int kb = ic->swept() ? 1 : ic->blk ? (int)ic->blocks.b.steps.size() : (int)ic->bwd_launch.size();
             timed("ic_forward", ZL * (4 + lb) + (N + 1) * 4 + 2 * N * sb, kf,
                   [&] { ic->apply_fwd(w.r.get(), dst, s); });
             timed("ic_backward", ZL * (4 + lb) + (N + 1) * 4 + N * lb + 2 * N * sb,

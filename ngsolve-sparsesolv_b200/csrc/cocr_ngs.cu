@@ -211,17 +211,6 @@ k_ngs_update(int n, S* __restrict__ x, const S* __restrict__ p, const S* __restr
     }
 }
 
-__global__ void k_ngs_loop_ctl(KState* st, cudaGraphConditionalHandle h, int use_cond) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    if (!st->done) {
-        st->it++;
-        if (st->it >= st->maxiter) { st->done = 1; st->iters = st->maxiter; }  // :368
-    }
-    st->loops++;
-    if (!st->done && st->loops >= st->max_loops) { st->done = 1; st->status = SSV_ERR_TIMEOUT; }
-    if (use_cond) cudaGraphSetConditional(h, st->done ? 0u : 1u);
-}
-
 struct CocrCtx {
     KrylovWork<double> w_d;
     KrylovWork<zdouble> w_z;
@@ -244,6 +233,15 @@ template <typename S>
 static void apply_pre(ssv_precond* pre, const S* x, S* y, const KState* st, int n, cudaStream_t s) {
     if (pre) precond_apply_any<S>(pre, x, y, st, s);
     else launch_k(k_copy<S>, grid_for(n, kBlock), kBlock, s, n, x, y);
+}
+
+// kernels of one application, where they are few (loop_unroll)
+static int pre_kernels(const ssv_precond* pre) {
+    if (!pre) return 1;
+    const bool real = pre->A->dtype == SSV_F64;
+    if (pre->kind == 1) return 2 + (real ? pre->ic_d.kernels_per_apply() : pre->ic_z.kernels_per_apply());
+    if (pre->kind == 4 && (real ? pre->sgs_d.swept() : pre->sgs_z.swept())) return 4;
+    return 1 << 20;
 }
 
 static std::string pre_key(const ssv_precond* pre) {
@@ -294,7 +292,7 @@ static void run_cocr_ngs(ssv_matrix* A, ssv_precond* pre, const uint8_t* fd, int
     const int dev_hist = printrates ? std::max(maxiter, 0) + 2 : 1;
     w.ensure(n, dev_hist);
     const RedBuf red = w.red();
-    const int g = grid_for(n, kBlock);
+    const int g = grid_vec(n);
     const S* v = reinterpret_cast<const S*>(A->val.get());
     S *x = d_x, *r = w.r.get(), *rt = w.z.get(), *p = w.p.get(), *q = w.Ap.get(), *qt = w.qt.get(),
       *t = w.t.get();
@@ -344,10 +342,9 @@ static void run_cocr_ngs(ssv_matrix* A, ssv_precond* pre, const uint8_t* fd, int
                     default: launch_k(k_ngs_spmv_dot<S, 32>, gg, kBlock, s, n, A->rp.get(), A->ci.get(), v, rt, t, fd, dst, red);
                 }
             }
-            launch_k(k_cocr_pq<S>, g, kBlock, s, n, rt, t, p, q, dst);
-            k_ngs_loop_ctl<<<1, 32, 0, s>>>(dst, hc, use_cond);
+            launch_k(k_cocr_pq<S>, g, kBlock, s, n, rt, t, p, q, dst, LoopCtl{hc, 1, use_cond, 0});
             SSV_LAUNCH_CHECK();
-        });
+        }, loop_unroll(pre_kernels(pre)));
     };
     std::vector<double> hs;  // printrates: the residual history over every cycle
     int used = 0, cycles = 0;
@@ -453,7 +450,7 @@ static void run_pcg(ssv_matrix* A, ssv_precond* pre, const uint8_t* fd, const ss
     const int dev_hist = cfg.save_residual_history ? std::max(cfg.max_iterations, 0) + 2 : 1;
     w.ensure(n, dev_hist);
     const RedBuf red = w.red();
-    const int g = grid_for(n, kBlock);
+    const int g = grid_vec(n);
     int64_t nk = 0;
     const S* v = reinterpret_cast<const S*>(A->val.get());
     if (fd) {
@@ -520,10 +517,9 @@ static void run_pcg(ssv_matrix* A, ssv_precond* pre, const uint8_t* fd, const ss
                                            w.r.get(), dst, red);
         if (pre) apply_pre<S>(pre, w.r.get(), w.z.get(), dst, n, s);
         launch_k(k_dot<S>, g, kBlock, s, n, w.r.get(), z, cfg.conjugate, dst, RED_CG_BETA, red, nullptr);
-        launch_k(k_pupdate<S>, g, kBlock, s, n, z, w.p.get(), dst);
-        k_loop_ctl<<<1, 32, 0, s>>>(dst, hc, use_cond);
+        launch_k(k_pupdate<S>, g, kBlock, s, n, z, w.p.get(), dst, LoopCtl{hc, 1, use_cond, 1});
         SSV_LAUNCH_CHECK();
-    });
+    }, loop_unroll(pre_kernels(pre)));
     SSV_CUDA(cudaStreamSynchronize(s));
     const double t1 = wall_seconds();
     if (cfg.max_iterations > 0) run_graph_loop(ctx.pcg_loop, dst, cfg.max_iterations);

@@ -404,12 +404,49 @@ k_cocr_update(int n, S* xb0, S* xb1, S* xb2, const S* __restrict__ p, const S* _
     }
 }
 
-// p = z + beta p (cg_solver.hpp:493-495)
+// Loop control, part of the iteration's last kernel (a launch of its own cost 3 us of
+// a small solve's 14 us between iterations): advance `iter`, stop at maxiter
+// (cg_solver.hpp:498-500; sparsesolv_solvers.hpp:368, which keeps no norm), enforce
+// the loop guard, and steer the graph's WHILE node when one is used.
+struct LoopCtl {
+    cudaGraphConditionalHandle h;
+    int on;     // 0: no loop control (the kernel outside an iteration)
+    int cond;   // a WHILE node is steered
+    int norm;   // the residual norm goes into the result at maxiter
+};
+
+__device__ inline void loop_step(KState* st, const LoopCtl& c) {
+    if (!st->done) {
+        st->it++;
+        if (st->it >= st->maxiter) {
+            st->done = 1;
+            st->iters = st->maxiter;
+            if (c.norm) {
+                st->converged = 0;
+                st->final_norm = st->norm_r;
+            }
+        }
+    }
+    st->loops++;
+    if (!st->done && st->loops >= st->max_loops) {
+        st->done = 1;
+        st->status = SSV_ERR_TIMEOUT;
+    }
+    if (c.cond) cudaGraphSetConditional(c.h, st->done ? 0u : 1u);
+}
+
+// p = z + beta p (cg_solver.hpp:493-495). A block that starts after the first one has
+// ended the loop at maxiter skips its part of p, which nothing reads any more.
 template <typename S>
 __global__ void __launch_bounds__(kBlock)
-k_pupdate(int n, const S* __restrict__ z, S* __restrict__ p, const KState* st) {
+k_pupdate(int n, const S* __restrict__ z, S* __restrict__ p, KState* st, LoopCtl ctl) {
     pdl_gate();
-    if (st->done) return;
+    const bool done = st->done != 0;
+    if (ctl.on && blockIdx.x == 0) {
+        __syncthreads();  // the block has read the flag
+        if (threadIdx.x == 0) loop_step(st, ctl);
+    }
+    if (done) return;
     const S beta = s_from2<S>(st->beta);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         p[i] = ST<S>::fma(beta, p[i], z[i]);
@@ -419,20 +456,20 @@ k_pupdate(int n, const S* __restrict__ z, S* __restrict__ p, const KState* st) {
 template <typename S>
 __global__ void __launch_bounds__(kBlock)
 k_cocr_pq(int n, const S* __restrict__ rt, const S* __restrict__ t, S* __restrict__ p,
-          S* __restrict__ q, const KState* st) {
+          S* __restrict__ q, KState* st, LoopCtl ctl) {
     pdl_gate();
-    if (st->done) return;
+    const bool done = st->done != 0;
+    if (ctl.on && blockIdx.x == 0) {
+        __syncthreads();
+        if (threadIdx.x == 0) loop_step(st, ctl);
+    }
+    if (done) return;
     const S beta = s_from2<S>(st->beta);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         p[i] = ST<S>::fma(beta, p[i], rt[i]);
         q[i] = ST<S>::fma(beta, q[i], t[i]);
     }
 }
-
-// Loop control, last node of the iteration body: advance `iter`, stop at
-// maxiter (cg_solver.hpp:498-500), enforce the loop guard, and steer the
-// graph's WHILE node when one is used.
-__global__ void k_loop_ctl(KState* st, cudaGraphConditionalHandle h, int use_cond);
 
 // ---------------------------------------------------------------------------
 // Vector helpers

@@ -100,6 +100,7 @@ template <typename S>
 __global__ void __launch_bounds__(kBlock)
 k_mrtr_dots(int n, S* __restrict__ Ard, const S* __restrict__ u, const S* __restrict__ rd,
             const S* __restrict__ y, KState* st, double2* partials, unsigned int* ticket) {
+    pdl_gate();
     if (st->done) return;
     const bool conj = st->conj != 0;
     double2 p0 = make_double2(0, 0), p1 = p0, p2 = p0;
@@ -164,8 +165,12 @@ k_mrtr_dots(int n, S* __restrict__ Ard, const S* __restrict__ u, const S* __rest
 template <typename S>
 __global__ void __launch_bounds__(kBlock)
 k_mrtr_update(int n, S* xb0, S* xb1, S* xb2, const S* __restrict__ u, const S* __restrict__ Ard,
-              S* __restrict__ p, S* __restrict__ y, S* __restrict__ rd, KState* st, RedBuf red) {
-    if (st->done) return;
+              S* __restrict__ p, S* __restrict__ y, S* __restrict__ rd, KState* st, RedBuf red, LoopCtl ctl) {
+    pdl_gate();
+    if (st->done) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) loop_step(st, ctl);
+        return;
+    }
     const int cur = st->cur;
     int nxt = cur;
     if (st->save_best) {
@@ -188,7 +193,10 @@ k_mrtr_update(int n, S* xb0, S* xb1, S* xb2, const S* __restrict__ u, const S* _
         part.x += ST<S>::norm2(ri);
     }
     double2 total;
-    if (grid_reduce2(part, red.partials, red.ticket, total)) dev_check(st, sqrt(total.x), 0, nxt);
+    if (grid_reduce2(part, red.partials, red.ticket, total)) {
+        dev_check(st, sqrt(total.x), 0, nxt);
+        loop_step(st, ctl);
+    }
 }
 
 template <typename S>
@@ -298,7 +306,7 @@ void run_mrtr(ssv_solver* sv, const ssv_config& cfg, const S* d_b, S* d_x, ssv_r
         P.D.alloc(n); P.iD.alloc(n);
         P.built = true;
     }
-    const int g = grid_for(n, kBlock);
+    const int g = grid_vec(n);
     KrylovWork<S>& w = mwork_of<S>(sv);
     const int dev_hist = cfg.save_residual_history ? std::max(cfg.max_iterations, 0) + 2 : 1;
     w.ensure(n, dev_hist);
@@ -406,13 +414,12 @@ void run_mrtr(ssv_solver* sv, const ssv_config& cfg, const S* d_b, S* d_x, ssv_r
     build_graph_loop(sv->loop, key, [&](cudaGraphConditionalHandle hc, int use_cond) {
         backward(P.rd.get(), P.u.get(), dst);
         forward(P.rd.get(), P.u.get(), P.Ard.get(), dst);
-        k_mrtr_dots<S><<<g, kBlock, 0, s>>>(n, P.Ard.get(), P.u.get(), P.rd.get(), P.y.get(), dst, w.partials.get(),
-                                           w.ticket.get());
-        k_mrtr_update<S><<<g, kBlock, 0, s>>>(n, w.xb[0].get(), w.xb[1].get(), w.xb[2].get(), P.u.get(),
-                                             P.Ard.get(), w.p.get(), P.y.get(), P.rd.get(), dst, red);
-        k_loop_ctl<<<1, 32, 0, s>>>(dst, hc, use_cond);
+        launch_k(k_mrtr_dots<S>, g, kBlock, s, n, P.Ard.get(), P.u.get(), P.rd.get(), P.y.get(), dst, w.partials.get(),
+                 w.ticket.get());
+        launch_k(k_mrtr_update<S>, g, kBlock, s, n, w.xb[0].get(), w.xb[1].get(), w.xb[2].get(), P.u.get(), P.Ard.get(),
+                 w.p.get(), P.y.get(), P.rd.get(), dst, red, LoopCtl{hc, 1, use_cond, 1});
         SSV_LAUNCH_CHECK();
-    });
+    }, loop_unroll(P.swept() ? 4 : 1 << 20));
     if (!h.done) run_graph_loop(sv->loop, dst, cfg.max_iterations);
     SSV_CUDA(cudaMemcpyAsync(&h, dst, sizeof(h), cudaMemcpyDeviceToHost, s));
     SSV_CUDA(cudaStreamSynchronize(s));

@@ -46,6 +46,10 @@ inline void launch_k(void (*k)(KArgs...), dim3 grid, dim3 block, cudaStream_t s,
 // (small copies: one cudaMemcpyAsync); ordered after the work queued on s.
 void h2d_staged(void* dst, const void* src, size_t bytes, cudaStream_t s);
 
+// Blocks of the vector kernels: four entries a thread at least, so that the last block of a
+// reduction has few partial sums to add up (262,144 doubles: 256 blocks in place of 1024).
+inline int grid_vec(int n) { return grid_for((n + 3) / 4, kBlock); }
+
 // Sub-warp width of the CSR kernels from the mean row length.
 int pick_lanes(double nnz_per_row);
 // SpMV launch shape: lanes | (rows per row group and pass) << 8
@@ -139,8 +143,14 @@ inline void abandon_capture(cudaStream_t s) {
     cudaGetLastError();
 }
 
+// Iterations in one body of the graph's WHILE node. Between two bodies 6 to 8 us pass in
+// which nothing runs; after the last iteration the rest of its body runs as kernels that
+// see the finished state and return, 1 to 2 us each. Four iterations a body pay where an
+// iteration has few kernels (`kernels` of the preconditioner), not with a multigrid cycle.
+inline int loop_unroll(int kernels) { return kernels <= 32 ? 4 : 1; }
+
 template <typename F>
-void build_graph_loop_body(GraphLoop& g, cudaStream_t s, F& body) {
+void build_graph_loop_body(GraphLoop& g, cudaStream_t s, F& body, int unroll) {
     if (graph_while_mode()) {
         SSV_CUDA(cudaGraphCreate(&g.graph, 0));
         cudaGraphConditionalHandle h;
@@ -155,9 +165,10 @@ void build_graph_loop_body(GraphLoop& g, cudaStream_t s, F& body) {
         cudaGraph_t bodyg = cp.conditional.phGraph_out[0];
         SSV_CUDA(cudaStreamBeginCaptureToGraph(s, bodyg, nullptr, nullptr, 0,
                                                cudaStreamCaptureModeThreadLocal));
-        body(h, 1);
+        for (int u = 0; u < unroll; ++u) body(h, 1);
         SSV_CUDA(cudaStreamEndCapture(s, &bodyg));
         SSV_CUDA(cudaGraphGetNodes(bodyg, nullptr, &g.body_nodes));
+        g.body_nodes /= (size_t)unroll;
         SSV_CUDA(cudaGraphInstantiate(&g.exec, g.graph, 0));
         g.cond = true;
     } else {
@@ -172,13 +183,13 @@ void build_graph_loop_body(GraphLoop& g, cudaStream_t s, F& body) {
 }
 
 template <typename F>
-void build_graph_loop(GraphLoop& g, const std::string& key_in, F&& body) {
+void build_graph_loop(GraphLoop& g, const std::string& key_in, F&& body, int unroll = 1) {
     const std::string key = key_in + (graph_while_mode() ? "|while" : "|chunk");
     if (g.exec && g.key == key) return;
     g.reset();
     cudaStream_t s = stream();
     try {
-        build_graph_loop_body(g, s, body);
+        build_graph_loop_body(g, s, body, unroll);
     } catch (...) {  // a failure inside the body (an allocation, a refused argument)
         abandon_capture(s);
         g.reset();

@@ -59,25 +59,6 @@ void GraphLoop::reset() {
     key.clear();
 }
 
-__global__ void k_loop_ctl(KState* st, cudaGraphConditionalHandle h, int use_cond) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    if (!st->done) {
-        st->it++;
-        if (st->it >= st->maxiter) {
-            st->done = 1;
-            st->converged = 0;
-            st->iters = st->maxiter;
-            st->final_norm = st->norm_r;
-        }
-    }
-    st->loops++;
-    if (!st->done && st->loops >= st->max_loops) {
-        st->done = 1;
-        st->status = SSV_ERR_TIMEOUT;
-    }
-    if (use_cond) cudaGraphSetConditional(h, st->done ? 0u : 1u);
-}
-
 // Cap on the executed loop bodies of every device-looped solve: maxiter + 4
 // (a loop that outruns its own iteration count means a stuck state), or the
 // process-wide override of ssv_set_loop_guard (> 0). A solve that reaches it
@@ -627,7 +608,7 @@ static void run_krylov(ssv_solver* sv, int method, const ssv_config& cfg, const 
     const int dev_hist = cfg.save_residual_history ? std::max(cfg.max_iterations, 0) + 2 : 1;
     w.ensure(n, dev_hist);
     const RedBuf red = w.red();
-    const int g = grid_for(n, kBlock);
+    const int g = grid_vec(n);
 
     // b and x into the working numbering, constrained entries zeroed
     if (perm) {
@@ -709,10 +690,9 @@ static void run_krylov(ssv_solver* sv, int method, const ssv_config& cfg, const 
                                                w.Ap.get(), w.r.get(), dst, red);
             if (ic) ic->apply(w.r.get(), w.z.get(), dst, s);
             launch_k(k_dot<S>, g, kBlock, s, n, w.r.get(), z, cfg.conjugate, dst, RED_CG_BETA, red, nullptr);
-            launch_k(k_pupdate<S>, g, kBlock, s, n, z, w.p.get(), dst);
-            k_loop_ctl<<<1, 32, 0, s>>>(dst, hc, use_cond);
+            launch_k(k_pupdate<S>, g, kBlock, s, n, z, w.p.get(), dst, LoopCtl{hc, 1, use_cond, 1});
             SSV_LAUNCH_CHECK();
-        });
+        }, loop_unroll(ic ? ic->kernels_per_apply() : 0));
     } else {  // COCR without preconditioner (sparsesolv_solvers.hpp:120-123)
         S* rt = w.z.get();
         S* q = w.Ap.get();
@@ -732,10 +712,9 @@ static void run_krylov(ssv_solver* sv, int method, const ssv_config& cfg, const 
                                                  q, w.r.get(), rt, dst, red);
             launch_spmv<S, S, 3>(lanes, n, wrp, wci, wv, rt, w.t.get(), nullptr, nullptr, dst, RED_COCR_BETA,
                                  red, nullptr, s);
-            launch_k(k_cocr_pq<S>, g, kBlock, s, n, rt, w.t.get(), w.p.get(), q, dst);
-            k_loop_ctl<<<1, 32, 0, s>>>(dst, hc, use_cond);
+            launch_k(k_cocr_pq<S>, g, kBlock, s, n, rt, w.t.get(), w.p.get(), q, dst, LoopCtl{hc, 1, use_cond, 1});
             SSV_LAUNCH_CHECK();
-        });
+        }, loop_unroll(0));
     }
     if (cfg.max_iterations > 0) run_graph_loop(sv->loop, dst, cfg.max_iterations);
     SSV_CUDA(cudaMemcpyAsync(&h, dst, sizeof(h), cudaMemcpyDeviceToHost, s));
@@ -835,7 +814,7 @@ static void profile_krylov(ssv_solver* sv, int method, const ssv_config& cfg, in
     SSV_CUDA(cudaMemcpyAsync(pst.get(), &h, sizeof(h), cudaMemcpyHostToDevice, s));
     KState* dst = pst.get();
     const RedBuf red = w.red();
-    const int g = grid_for(n, kBlock);
+    const int g = grid_vec(n);
     cudaEvent_t e0, e1;
     SSV_CUDA(cudaEventCreate(&e0));
     SSV_CUDA(cudaEventCreate(&e1));
@@ -878,7 +857,7 @@ static void profile_krylov(ssv_solver* sv, int method, const ssv_config& cfg, in
         timed("dot_beta", 2 * N * sb, 1, [&] {
             launch_k(k_dot<S>, g, kBlock, s, n, w.r.get(), z, cfg.conjugate, dst, RED_CG_BETA, red, nullptr);
         });
-        timed("p_update", 3 * N * sb, 1, [&] { launch_k(k_pupdate<S>, g, kBlock, s, n, z, w.p.get(), dst); });
+        timed("p_update", 3 * N * sb, 1, [&] { launch_k(k_pupdate<S>, g, kBlock, s, n, z, w.p.get(), dst, LoopCtl{}); });
     } else if (method == SSV_METHOD_COCR) {
         S* rt = w.z.get();
         S* q = w.Ap.get();
@@ -893,7 +872,7 @@ static void profile_krylov(ssv_solver* sv, int method, const ssv_config& cfg, in
             launch_spmv<S, S, 3>(lanes, n, wrp, wci, wv, rt, w.t.get(), nullptr, nullptr, dst, RED_COCR_BETA, red,
                                  nullptr, s);
         });
-        timed("pq_update", 6 * N * sb, 1, [&] { launch_k(k_cocr_pq<S>, g, kBlock, s, n, rt, w.t.get(), w.p.get(), q, dst); });
+        timed("pq_update", 6 * N * sb, 1, [&] { launch_k(k_cocr_pq<S>, g, kBlock, s, n, rt, w.t.get(), w.p.get(), q, dst, LoopCtl{}); });
     } else {
         fail(SSV_ERR_INVALID_ARG, "ssv_solver_profile: method not profiled");
     }

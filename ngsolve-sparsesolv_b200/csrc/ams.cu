@@ -92,6 +92,13 @@ __device__ __forceinline__ void load_row(const float* __restrict__ p, float (&o)
     }
 }
 
+// Kernels of one or two columns read their first entries before the gate. With blocks of
+// columns several cycles run side by side (the frequencies of a batch), and blocks that
+// wait with their entries in registers only take room from the others' work: six cycles of
+// eight columns 89 -> 95 ms a solve.
+template <int NV>
+constexpr bool kReadAhead = NV <= 2;
+
 template <typename A, typename B>
 using wider_t = std::conditional_t<(sizeof(A) >= sizeof(B)), A, B>;
 
@@ -105,36 +112,61 @@ template <typename TV, typename TX, typename TY, int NV, int LANES, int MODE, bo
 __global__ void __launch_bounds__(kBlock)
 k_mv_spmv(int n, const int* __restrict__ rp, const int* __restrict__ ci, const TV* __restrict__ v,
           const TX* __restrict__ x, TY* __restrict__ y, const TY* __restrict__ b, const TY* __restrict__ d, TY w,
-          const KState* st) {
+          const uint8_t* __restrict__ fd, const KState* st) {
     using TA = wider_t<TV, TX>;
-    pdl_gate();
-    if (st && st->done) return;
     const int sub = threadIdx.x % LANES;
     const int rpb = kBlock / LANES;
     const int lane_row = (threadIdx.x & 31) / LANES;  // warp-uniform trip count
-    for (int row0 = blockIdx.x * rpb * U + threadIdx.x / LANES; row0 - lane_row < n; row0 += gridDim.x * rpb * U) {
-        int kk[U], ke[U];
-        TA acc[U][NV];
+    int kk[U], ke[U], col[U];
+    TA a[U];
+    // row pointers and first entries of a group of rows
+    auto head = [&](int r0) {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const int row = row0 + u * rpb;
+            const int row = r0 + u * rpb;
             kk[u] = row < n ? rp[row] + sub : 0;
             ke[u] = row < n ? rp[row + 1] : 0;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const bool on = kk[u] < ke[u];
+            a[u] = on ? (TA)v[kk[u]] : TA(0);
+            col[u] = on ? ci[kk[u]] : -1;
+        }
+    };
+    int row0 = blockIdx.x * rpb * U + threadIdx.x / LANES;
+    if constexpr (!kReadAhead<NV>) {
+        pdl_gate();
+        if (st && st->done) return;
+    }
+    head(row0);
+    if constexpr (kReadAhead<NV>) {
+        pdl_gate();
+        if (st && st->done) return;
+    }
+    for (; row0 - lane_row < n; row0 += gridDim.x * rpb * U) {
+        TA acc[U][NV];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
 #pragma unroll
             for (int c = 0; c < NV; ++c) acc[u][c] = TA(0);
-        }
         while (true) {
-            TA a[U];
-            int col[U];
             bool any = false;
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const bool on = kk[u] < ke[u];
-                a[u] = on ? (TA)v[kk[u]] : TA(0);
-                col[u] = on ? ci[kk[u]] : -1;
-                any |= on;
-            }
+            for (int u = 0; u < U; ++u) any |= col[u] >= 0;
             if (!any) break;
+            TA an[U];
+            int cn[U];
+            auto next = [&] {
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    kk[u] += LANES;
+                    const bool on = kk[u] < ke[u];
+                    an[u] = on ? (TA)v[kk[u]] : TA(0);
+                    cn[u] = on ? ci[kk[u]] : -1;
+                }
+            };
+            if constexpr (kReadAhead<NV>) next();  // on their way while these are gathered
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 if (col[u] >= 0) {
@@ -147,10 +179,16 @@ k_mv_spmv(int n, const int* __restrict__ rp, const int* __restrict__ ci, const T
                         load_row<NV>(x + (size_t)col[u] * NV, xv);
 #pragma unroll
                     for (int c = 0; c < NV; ++c) acc[u][c] += a[u] * (TA)xv[c];
-                    kk[u] += LANES;
                 }
             }
+            if constexpr (!kReadAhead<NV>) next();
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                a[u] = an[u];
+                col[u] = cn[u];
+            }
         }
+        if (row0 + (int)gridDim.x * rpb * U - lane_row < n) head(row0 + gridDim.x * rpb * U);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
 #pragma unroll
@@ -172,7 +210,8 @@ k_mv_spmv(int n, const int* __restrict__ rp, const int* __restrict__ ci, const T
                     } else {
                         const TY r = b[base + c] - ac;
                         const TY xo = (TY)x[base + c];
-                        y[base + c] = RECIP ? xo + r * d[row] : xo + r / d[row];
+                        const TY o = RECIP ? xo + r * d[row] : xo + r / d[row];
+                        y[base + c] = kReadAhead<NV> && fd && !fd[row] ? TY(0) : o;  // fd: the cycle's last sweep
                     }
                 }
             }
@@ -195,7 +234,8 @@ k_mv_spmv(int n, const int* __restrict__ rp, const int* __restrict__ ci, const T
 // the output of one row of a sliced-ELL product, by mode
 template <typename TX, typename TY, int NV, int MODE, bool RECIP, typename TA>
 __device__ __forceinline__ void sell_store(int row, const TA (&acc)[NV], const TX* __restrict__ x, TY* __restrict__ y,
-                                           const TY* __restrict__ b, const TY* __restrict__ d, TY w) {
+                                           const TY* __restrict__ b, const TY* __restrict__ d, TY w,
+                                           const uint8_t* __restrict__ fd) {
     const size_t base = (size_t)row * NV;
 #pragma unroll
     for (int c = 0; c < NV; ++c) {
@@ -209,7 +249,8 @@ __device__ __forceinline__ void sell_store(int row, const TA (&acc)[NV], const T
         } else {
             const TY r = b[base + c] - ac;
             const TY xo = (TY)x[base + c];
-            y[base + c] = RECIP ? xo + r * d[row] : xo + r / d[row];
+            const TY o = RECIP ? xo + r * d[row] : xo + r / d[row];
+            y[base + c] = kReadAhead<NV> && fd && !fd[row] ? TY(0) : o;  // fd: the cycle's last sweep
         }
     }
 }
@@ -218,13 +259,16 @@ template <typename TX, typename TY, int NV, int MODE, bool RECIP, int R, int P =
 __global__ void __launch_bounds__(kBlock)
 k_sell_spmv(int slices, const int* __restrict__ off, const int* __restrict__ rows, const int* __restrict__ ci,
             const double* __restrict__ v, const TX* __restrict__ x, TY* __restrict__ y, const TY* __restrict__ b,
-            const TY* __restrict__ d, TY w, const KState* st, int n) {
+            const TY* __restrict__ d, TY w, const uint8_t* __restrict__ fd, const KState* st, int n) {
     using TA = wider_t<double, TX>;
-    pdl_gate();
-    if (st && st->done) return;
     const int lane = threadIdx.x & 31;
     const int wpb = kBlock / 32;
-    for (int sl0 = (blockIdx.x * wpb + threadIdx.x / 32) * P; sl0 < slices; sl0 += gridDim.x * wpb * P) {
+    const int first = (blockIdx.x * wpb + threadIdx.x / 32) * P;
+    if constexpr (!kReadAhead<NV>) {
+        pdl_gate();
+        if (st && st->done) return;
+    }
+    for (int sl0 = first; sl0 < slices; sl0 += gridDim.x * wpb * P) {
         int e[P], e1[P], row[P];
         TA acc[P][NV];
         double a[P][R];
@@ -244,6 +288,10 @@ k_sell_spmv(int slices, const int* __restrict__ off, const int* __restrict__ row
                 a[q][u] = k < e1[q] ? v[k] : 0.0;
                 col[q][u] = k < e1[q] ? ci[k] : -1;
             }
+        }
+        if (kReadAhead<NV> && sl0 == first) {
+            pdl_gate();
+            if (st && st->done) return;
         }
         while (true) {
             bool any = false;
@@ -288,7 +336,7 @@ k_sell_spmv(int slices, const int* __restrict__ off, const int* __restrict__ row
         }
 #pragma unroll
         for (int q = 0; q < P; ++q)
-            if (row[q] >= 0) sell_store<TX, TY, NV, MODE, RECIP>(row[q], acc[q], x, y, b, d, w);
+            if (row[q] >= 0) sell_store<TX, TY, NV, MODE, RECIP>(row[q], acc[q], x, y, b, d, w, fd);
     }
 }
 
@@ -304,7 +352,7 @@ template <typename TX, typename TY, int NV, int MODE, bool RECIP, int R>
 __global__ void __launch_bounds__(kBlock)
 k_sell_spmv_cs(int slices, const int* __restrict__ off, const int* __restrict__ rows, const int* __restrict__ ci,
                const double* __restrict__ v, const TX* __restrict__ x, TY* __restrict__ y, const TY* __restrict__ b,
-               const TY* __restrict__ d, TY w, const KState* st, int n) {
+               const TY* __restrict__ d, TY w, const uint8_t*, const KState* st, int n) {
     static_assert(NV == 4 || NV == 8, "column-split form: 4 or 8 columns");
     constexpr int CS = 2;       // columns per lane
     constexpr int G = NV / CS;  // lanes per row
@@ -396,19 +444,18 @@ template <typename TX, typename TY, int NV, int MODE, bool RECIP, int R>
 __global__ void __launch_bounds__(kBlock)
 k_sell_spmv_deep(int slices, const int* __restrict__ off, const int* __restrict__ rows, const int* __restrict__ ci,
                  const double* __restrict__ v, const TX* __restrict__ x, TY* __restrict__ y, const TY* __restrict__ b,
-                 const TY* __restrict__ d, TY w, const KState* st, int n) {
+                 const TY* __restrict__ d, TY w, const uint8_t* __restrict__ fd, const KState* st, int n) {
     using TA = wider_t<double, TX>;
-    pdl_gate();
-    if (st && st->done) return;
     const int lane = threadIdx.x & 31;
     const int wpb = kBlock / 32;
+    const int first = blockIdx.x * wpb + threadIdx.x / 32;
     auto gather = [&](int c, TX (&o)[NV]) {
         if constexpr (MODE == MV_TWO)  // columns past the row count read the b slot
             load_row<NV>(c < n ? x + (size_t)c * NV : reinterpret_cast<const TX*>(b) + (size_t)(c - n) * NV, o);
         else
             load_row<NV>(x + (size_t)c * NV, o);
     };
-    for (int sl = blockIdx.x * wpb + threadIdx.x / 32; sl < slices; sl += gridDim.x * wpb) {
+    for (int sl = first; sl < slices; sl += gridDim.x * wpb) {
         const int e1 = off[sl + 1];
         int e = off[sl] + lane;
         const int row = rows[(size_t)sl * 32 + lane];
@@ -416,19 +463,26 @@ k_sell_spmv_deep(int slices, const int* __restrict__ off, const int* __restrict_
 #pragma unroll
         for (int c = 0; c < NV; ++c) acc[c] = TA(0);
         double a[R], an[R];
-        int cn[R];
+        int c0[R], cn[R];
         bool on[R];
         TX xv[R][NV];
 #pragma unroll
-        for (int u = 0; u < R; ++u) {  // round 0: values, columns, gathers; round 1: values, columns
+        for (int u = 0; u < R; ++u) {  // rounds 0 and 1: values, columns
             const int k = e + 32 * u;
             a[u] = k < e1 ? v[k] : 0.0;
-            const int c0 = k < e1 ? ci[k] : -1;
-            on[u] = c0 >= 0;
-            if (on[u]) gather(c0, xv[u]);
+            c0[u] = k < e1 ? ci[k] : -1;
             const int k1 = k + 32 * R;
             an[u] = k1 < e1 ? v[k1] : 0.0;
             cn[u] = k1 < e1 ? ci[k1] : -1;
+        }
+        if (sl == first) {
+            pdl_gate();
+            if (st && st->done) return;
+        }
+#pragma unroll
+        for (int u = 0; u < R; ++u) {  // round 0: gathers
+            on[u] = c0[u] >= 0;
+            if (on[u]) gather(c0[u], xv[u]);
         }
         while (e < e1) {
             double a2[R];
@@ -462,7 +516,7 @@ k_sell_spmv_deep(int slices, const int* __restrict__ off, const int* __restrict_
             }
             e += 32 * R;
         }
-        if (row >= 0) sell_store<TX, TY, NV, MODE, RECIP>(row, acc, x, y, b, d, w);
+        if (row >= 0) sell_store<TX, TY, NV, MODE, RECIP>(row, acc, x, y, b, d, w, fd);
     }
 }
 
@@ -473,28 +527,60 @@ __global__ void __launch_bounds__(kBlock)
 k_mv_pi_restrict(int n, const int* __restrict__ rp, const int* __restrict__ ci, const double* __restrict__ px,
                  const double* __restrict__ py, const double* __restrict__ pz, const double* __restrict__ r,
                  TO* __restrict__ ox, TO* __restrict__ oy, TO* __restrict__ oz, const KState* st) {
-    pdl_gate();
-    if (st && st->done) return;
     const int sub = threadIdx.x % LANES;
     const int rpb = kBlock / LANES;
     const int lane_row = (threadIdx.x & 31) / LANES;
-    for (int row = blockIdx.x * rpb + threadIdx.x / LANES; row - lane_row < n; row += gridDim.x * rpb) {
+    int row = blockIdx.x * rpb + threadIdx.x / LANES;
+    // entries are read one step ahead of their gathers, the first ones before the wait
+    int k = 0, k1 = 0, j = -1;
+    double vx = 0.0, vy = 0.0, vz = 0.0;
+    auto entry = [&] {
+        j = k < k1 ? ci[k] : -1;
+        if (j >= 0) {
+            vx = px[k];
+            vy = py[k];
+            vz = pz[k];
+        }
+    };
+    auto head = [&](int i) {
+        k = i < n ? rp[i] + sub : 0;
+        k1 = i < n ? rp[i + 1] : 0;
+        entry();
+    };
+    if constexpr (!kReadAhead<NV>) {
+        pdl_gate();
+        if (st && st->done) return;
+    }
+    head(row);
+    if constexpr (kReadAhead<NV>) {
+        pdl_gate();
+        if (st && st->done) return;
+    }
+    for (; row - lane_row < n; row += gridDim.x * rpb) {
         const bool valid = row < n;
         double ax[NV], ay[NV], az[NV];
 #pragma unroll
         for (int c = 0; c < NV; ++c) ax[c] = ay[c] = az[c] = 0.0;
-        if (valid)
-            for (int k = rp[row] + sub; k < rp[row + 1]; k += LANES) {
+        while (j >= 0) {
                 double rr[NV];
-                load_row<NV>(r + (size_t)ci[k] * NV, rr);
-                const double vx = px[k], vy = py[k], vz = pz[k];
+                load_row<NV>(r + (size_t)j * NV, rr);
+                const double ux = vx, uy = vy, uz = vz;
+                if constexpr (kReadAhead<NV>) {
+                    k += LANES;
+                    entry();
+                }
 #pragma unroll
                 for (int c = 0; c < NV; ++c) {
-                    ax[c] += vx * rr[c];
-                    ay[c] += vy * rr[c];
-                    az[c] += vz * rr[c];
+                    ax[c] += ux * rr[c];
+                    ay[c] += uy * rr[c];
+                    az[c] += uz * rr[c];
                 }
-            }
+                if constexpr (!kReadAhead<NV>) {
+                    k += LANES;
+                    entry();
+                }
+        }
+        if (row + (int)gridDim.x * rpb - lane_row < n) head(row + gridDim.x * rpb);
 #pragma unroll
         for (int o = LANES / 2; o > 0; o >>= 1)
 #pragma unroll
@@ -522,31 +608,61 @@ k_mv_pi_prolong(int n, const int* __restrict__ rp, const int* __restrict__ ci, c
                 const double* __restrict__ py, const double* __restrict__ pz, const TG* __restrict__ gx,
                 const TG* __restrict__ gy, const TG* __restrict__ gz, double* __restrict__ x, double w,
                 const KState* st) {
-    pdl_gate();
-    if (st && st->done) return;
     const int sub = threadIdx.x % LANES;
     const int rpb = kBlock / LANES;
     const int lane_row = (threadIdx.x & 31) / LANES;
-    for (int row = blockIdx.x * rpb + threadIdx.x / LANES; row - lane_row < n; row += gridDim.x * rpb) {
+    int row = blockIdx.x * rpb + threadIdx.x / LANES;
+    int k = 0, k1 = 0, j = -1;
+    double vx = 0.0, vy = 0.0, vz = 0.0;
+    auto entry = [&] {
+        j = k < k1 ? ci[k] : -1;
+        if (j >= 0) {
+            vx = px[k];
+            vy = py[k];
+            vz = pz[k];
+        }
+    };
+    auto head = [&](int i) {
+        k = i < n ? rp[i] + sub : 0;
+        k1 = i < n ? rp[i + 1] : 0;
+        entry();
+    };
+    if constexpr (!kReadAhead<NV>) {
+        pdl_gate();
+        if (st && st->done) return;
+    }
+    head(row);
+    if constexpr (kReadAhead<NV>) {
+        pdl_gate();
+        if (st && st->done) return;
+    }
+    for (; row - lane_row < n; row += gridDim.x * rpb) {
         const bool valid = row < n;
         double sx[NV], sy[NV], sz[NV];
 #pragma unroll
         for (int c = 0; c < NV; ++c) sx[c] = sy[c] = sz[c] = 0.0;
-        if (valid)
-            for (int k = rp[row] + sub; k < rp[row + 1]; k += LANES) {
-                const size_t j = (size_t)ci[k] * NV;
+        while (j >= 0) {
                 TG vgx[NV], vgy[NV], vgz[NV];
-                load_row<NV>(gx + j, vgx);
-                load_row<NV>(gy + j, vgy);
-                load_row<NV>(gz + j, vgz);
-                const double vx = px[k], vy = py[k], vz = pz[k];
+                load_row<NV>(gx + (size_t)j * NV, vgx);
+                load_row<NV>(gy + (size_t)j * NV, vgy);
+                load_row<NV>(gz + (size_t)j * NV, vgz);
+                const double ux = vx, uy = vy, uz = vz;
+                if constexpr (kReadAhead<NV>) {
+                    k += LANES;
+                    entry();
+                }
 #pragma unroll
                 for (int c = 0; c < NV; ++c) {
-                    sx[c] += vx * (double)vgx[c];
-                    sy[c] += vy * (double)vgy[c];
-                    sz[c] += vz * (double)vgz[c];
+                    sx[c] += ux * (double)vgx[c];
+                    sy[c] += uy * (double)vgy[c];
+                    sz[c] += uz * (double)vgz[c];
                 }
-            }
+                if constexpr (!kReadAhead<NV>) {
+                    k += LANES;
+                    entry();
+                }
+        }
+        if (row + (int)gridDim.x * rpb - lane_row < n) head(row + gridDim.x * rpb);
 #pragma unroll
         for (int o = LANES / 2; o > 0; o >>= 1)
 #pragma unroll
@@ -641,6 +757,56 @@ __global__ void k_mv_mask_copy(int n, const TI* __restrict__ in, const uint8_t* 
     }
 }
 
+// sum_k row[k] src[k] over k = k0 + lane, k0 + lane + 32, ... < k1, the first kDenseAhead
+// entries of the lane passed in (read before the launch's wait for its first row)
+constexpr int kDenseAhead = 8;
+__device__ __forceinline__ void dense_ahead(const double* __restrict__ lr, int k, int k1, double (&m)[kDenseAhead]) {
+#pragma unroll
+    for (int u = 0; u < kDenseAhead; ++u) m[u] = k + 32 * u < k1 ? lr[k + 32 * u] : 0.0;
+}
+template <typename T, int NV>
+__device__ __forceinline__ void dense_row(const double* __restrict__ lr, const T* src, int k, int k1,
+                                          const double (&m)[kDenseAhead], double (&acc)[NV]) {
+#pragma unroll
+    for (int c = 0; c < NV; ++c) acc[c] = 0.0;
+    // (loads without a branch each, so that they are in flight together)
+    if constexpr (kReadAhead<NV>) {
+        T g[kDenseAhead][NV];
+#pragma unroll
+        for (int u = 0; u < kDenseAhead; ++u) load_row<NV>(src + (size_t)min(k + 32 * u, k1 - 1) * NV, g[u]);
+#pragma unroll
+        for (int u = 0; u < kDenseAhead; ++u)
+#pragma unroll
+            for (int c = 0; c < NV; ++c) acc[c] += m[u] * (k + 32 * u < k1 ? (double)g[u][c] : 0.0);
+        k += 32 * kDenseAhead;
+    }
+    for (; k < k1; k += 32) {
+        const double a = lr[k];
+#pragma unroll
+        for (int c = 0; c < NV; ++c) acc[c] += a * (double)src[(size_t)k * NV + c];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int c = 0; c < NV; ++c) acc[c] += __shfl_down_sync(0xffffffffu, acc[c], o);
+}
+
+// The cycle's start: b0 = mask ? in : 0 and the first Jacobi sweep from x = 0 on it
+template <int NV, bool RECIP>
+__global__ void __launch_bounds__(kBlock)
+k_mv_mask_sweep(int n, const double* __restrict__ in, const uint8_t* __restrict__ fd, const double* __restrict__ d,
+                double* __restrict__ b0, double* __restrict__ x, const KState* st) {
+    pdl_gate();
+    if (st && st->done) return;
+    const int64_t total = (int64_t)n * NV;
+    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total; q += (int64_t)gridDim.x * blockDim.x) {
+        const int i = (int)(q / NV);
+        const double b = (!fd || fd[i]) ? in[q] : 0.0;
+        b0[q] = b;
+        x[q] = RECIP ? b * d[i] : b / d[i];
+    }
+}
+
 // Coarsest solve x = L^{-T} (D^+ (L^{-1} b)) (the LDL^T pseudo-inverse kept
 // factored), FP64 factors and FP64 accumulation in both forms; warp per row.
 // Forward part: z_i = (sum_{k<=i} Linv[i][k] b_k) / d_i, or 0 for a dropped
@@ -649,23 +815,17 @@ template <typename T, int NV>
 __global__ void __launch_bounds__(kBlock)
 k_mv_coarse_fwd(int n, const double* __restrict__ Li, const double* __restrict__ piv, const T* __restrict__ b,
                 double* __restrict__ z, const KState* st) {
+    const int lane = threadIdx.x & 31;
+    const int first = blockIdx.x * (kBlock / 32) + threadIdx.x / 32;
+    double m[kDenseAhead];
+    if constexpr (kReadAhead<NV>) dense_ahead(Li + (size_t)first * n, lane, first < n ? first + 1 : 0, m);
     pdl_gate();
     if (st && st->done) return;
-    const int lane = threadIdx.x & 31;
-    for (int row = blockIdx.x * (kBlock / 32) + threadIdx.x / 32; row < n; row += gridDim.x * (kBlock / 32)) {
-        double acc[NV];
-#pragma unroll
-        for (int c = 0; c < NV; ++c) acc[c] = 0.0;
+    for (int row = first; row < n; row += gridDim.x * (kBlock / 32)) {
         const double* lr = Li + (size_t)row * n;
-        for (int k = lane; k <= row; k += 32) {
-            const double a = lr[k];
-#pragma unroll
-            for (int c = 0; c < NV; ++c) acc[c] += a * (double)b[(size_t)k * NV + c];
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-            for (int c = 0; c < NV; ++c) acc[c] += __shfl_down_sync(0xffffffffu, acc[c], o);
+        if (kReadAhead<NV> && row != first) dense_ahead(lr, lane, row + 1, m);
+        double acc[NV];
+        dense_row<T, NV>(lr, b, lane, row + 1, m, acc);
         if (lane == 0) {
             const double d = piv[row];
 #pragma unroll
@@ -679,23 +839,17 @@ template <typename T, int NV>
 __global__ void __launch_bounds__(kBlock)
 k_mv_coarse_bwd(int n, const double* __restrict__ LiT, const double* __restrict__ z, T* __restrict__ x,
                 const KState* st) {
+    const int lane = threadIdx.x & 31;
+    const int first = blockIdx.x * (kBlock / 32) + threadIdx.x / 32;
+    double m[kDenseAhead];
+    if constexpr (kReadAhead<NV>) dense_ahead(LiT + (size_t)first * n, first + lane, first < n ? n : 0, m);
     pdl_gate();
     if (st && st->done) return;
-    const int lane = threadIdx.x & 31;
-    for (int row = blockIdx.x * (kBlock / 32) + threadIdx.x / 32; row < n; row += gridDim.x * (kBlock / 32)) {
-        double acc[NV];
-#pragma unroll
-        for (int c = 0; c < NV; ++c) acc[c] = 0.0;
+    for (int row = first; row < n; row += gridDim.x * (kBlock / 32)) {
         const double* lr = LiT + (size_t)row * n;
-        for (int k = row + lane; k < n; k += 32) {
-            const double a = lr[k];
-#pragma unroll
-            for (int c = 0; c < NV; ++c) acc[c] += a * z[(size_t)k * NV + c];
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-            for (int c = 0; c < NV; ++c) acc[c] += __shfl_down_sync(0xffffffffu, acc[c], o);
+        if (kReadAhead<NV> && row != first) dense_ahead(lr, row + lane, n, m);
+        double acc[NV];
+        dense_row<double, NV>(lr, z, row + lane, n, m, acc);
         if (lane == 0)
 #pragma unroll
             for (int c = 0; c < NV; ++c) x[(size_t)row * NV + c] = (T)acc[c];
@@ -726,8 +880,6 @@ struct Tri {
 template <typename T, int NV, int LANES, int MODE, bool RECIP, int K = 3>
 __global__ void __launch_bounds__(kBlock)
 k_mv3_spmv(Tri<T, K> t, T w, const KState* st) {
-    pdl_gate();
-    if (st && st->done) return;
     const int q = blockIdx.y;
     const int n = t.n[q];
     const int* __restrict__ rp = t.rp[q];
@@ -740,25 +892,57 @@ k_mv3_spmv(Tri<T, K> t, T w, const KState* st) {
     const int sub = threadIdx.x % LANES;
     const int rpb = kBlock / LANES;
     const int lane_row = (threadIdx.x & 31) / LANES;
-    for (int row = blockIdx.x * rpb + threadIdx.x / LANES; row - lane_row < n; row += gridDim.x * rpb) {
+    int row = blockIdx.x * rpb + threadIdx.x / LANES;
+    // a row's first entries are read together, before the gate for the first row
+    constexpr int A = NV == 1 ? 4 : NV == 2 ? 2 : 1;
+    int k = 0, k1 = 0, j[A];
+    T a[A];
+    auto head = [&](int i) {
+        k = i < n ? rp[i] + sub : 0;
+        k1 = i < n ? rp[i + 1] : 0;
+#pragma unroll
+        for (int u = 0; u < A; ++u) {
+            j[u] = k + u * LANES < k1 ? ci[k + u * LANES] : -1;
+            if (j[u] >= 0) a[u] = v[k + u * LANES];
+        }
+    };
+    if constexpr (!kReadAhead<NV>) {
+        pdl_gate();
+        if (st && st->done) return;
+    }
+    head(row);
+    if constexpr (kReadAhead<NV>) {
+        pdl_gate();
+        if (st && st->done) return;
+    }
+    for (; row - lane_row < n; row += gridDim.x * rpb) {
         const bool valid = row < n;
         T acc[NV];
 #pragma unroll
         for (int c = 0; c < NV; ++c) acc[c] = T(0);
-        if (valid) {
-            const int k1 = rp[row + 1];
-            for (int k = rp[row] + sub; k < k1; k += LANES) {
-                const T a = v[k];
-                const int j = ci[k];
-                T xv[NV];
-                if constexpr (MODE == MV_TWO)
-                    load_row<NV>(j < n ? x + (size_t)j * NV : b + (size_t)(j - n) * NV, xv);
-                else
-                    load_row<NV>(x + (size_t)j * NV, xv);
+        auto gather = [&](int i, T (&o)[NV]) {
+            if constexpr (MODE == MV_TWO)
+                load_row<NV>(i < n ? x + (size_t)i * NV : b + (size_t)(i - n) * NV, o);
+            else
+                load_row<NV>(x + (size_t)i * NV, o);
+        };
+        T g[A][NV];
 #pragma unroll
-                for (int c = 0; c < NV; ++c) acc[c] += a * xv[c];
-            }
+        for (int u = 0; u < A; ++u)
+            if (j[u] >= 0) gather(j[u], g[u]);
+#pragma unroll
+        for (int u = 0; u < A; ++u)
+            if (j[u] >= 0)
+#pragma unroll
+                for (int c = 0; c < NV; ++c) acc[c] += a[u] * g[u][c];
+        for (k += A * LANES; k < k1; k += LANES) {
+            const T ak = v[k];
+            T xv[NV];
+            gather(ci[k], xv);
+#pragma unroll
+            for (int c = 0; c < NV; ++c) acc[c] += ak * xv[c];
         }
+        if (row + (int)gridDim.x * rpb - lane_row < n) head(row + gridDim.x * rpb);
 #pragma unroll
         for (int o = LANES / 2; o > 0; o >>= 1)
 #pragma unroll
@@ -845,35 +1029,24 @@ struct TriCoarse {
 template <typename T, int NV, bool FWD, int K = 3>
 __global__ void __launch_bounds__(kBlock)
 k_mv3_coarse(TriCoarse<K> t, const KState* st) {
-    pdl_gate();
-    if (st && st->done) return;
     const int q = blockIdx.y;
     const int n = t.n[q];
+    const double* __restrict__ M = t.M[q];
     const int lane = threadIdx.x & 31;
-    for (int row = blockIdx.x * (kBlock / 32) + threadIdx.x / 32; row < n; row += gridDim.x * (kBlock / 32)) {
+    const int first = blockIdx.x * (kBlock / 32) + threadIdx.x / 32;
+    double m[kDenseAhead];
+    // forward rows end at the diagonal, backward ones start there
+    auto k0 = [&](int row) { return FWD ? lane : row + lane; };
+    auto k1 = [&](int row) { return FWD ? row + 1 : n; };
+    if constexpr (kReadAhead<NV>) dense_ahead(M + (size_t)first * n, k0(first), first < n ? k1(first) : 0, m);
+    pdl_gate();
+    if (st && st->done) return;
+    for (int row = first; row < n; row += gridDim.x * (kBlock / 32)) {
+        const double* lr = M + (size_t)row * n;
+        if (kReadAhead<NV> && row != first) dense_ahead(lr, k0(row), k1(row), m);
         double acc[NV];
-#pragma unroll
-        for (int c = 0; c < NV; ++c) acc[c] = 0.0;
-        const double* lr = t.M[q] + (size_t)row * n;
-        if constexpr (FWD) {
-            const T* b = (const T*)t.io[q];
-            for (int k = lane; k <= row; k += 32) {
-                const double a = lr[k];
-#pragma unroll
-                for (int c = 0; c < NV; ++c) acc[c] += a * (double)b[(size_t)k * NV + c];
-            }
-        } else {
-            const double* z = t.cz[q];
-            for (int k = row + lane; k < n; k += 32) {
-                const double a = lr[k];
-#pragma unroll
-                for (int c = 0; c < NV; ++c) acc[c] += a * z[(size_t)k * NV + c];
-            }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-            for (int c = 0; c < NV; ++c) acc[c] += __shfl_down_sync(0xffffffffu, acc[c], o);
+        if constexpr (FWD) dense_row<T, NV>(lr, (const T*)t.io[q], k0(row), k1(row), m, acc);
+        else dense_row<double, NV>(lr, t.cz[q], k0(row), k1(row), m, acc);
         if (lane == 0) {
             if constexpr (FWD) {
                 const double dd = t.piv[q][row];
@@ -909,13 +1082,13 @@ struct TailSet {
 // y = T b for K hierarchies (blockIdx.y), warp per row, FP64 accumulation
 template <typename T, int NV, int K>
 __global__ void __launch_bounds__(kBlock) k_tail_apply(TailSet<T, K> t, const KState* st) {
-    pdl_gate();
-    if (st && st->done) return;
     const int q = blockIdx.y;
     const int n = t.n[q];
     const double* __restrict__ M = t.M[q];
     const T* __restrict__ b = t.b[q];
     const int lane = threadIdx.x & 31;
+    pdl_gate();
+    if (st && st->done) return;
     for (int row = blockIdx.x * (kBlock / 32) + threadIdx.x / 32; row < n; row += gridDim.x * (kBlock / 32)) {
         double acc[NV];
 #pragma unroll
@@ -1263,10 +1436,11 @@ constexpr int kSellShapes[] = {2, 4, 8, kSellPair | 2, kSellPair | 4, kSellDeep 
 
 template <typename TV, typename TX, typename TY, int NV, int MODE, bool RECIP>
 static void launch_mv(int lanes, int u, int grid, cudaStream_t s, int n, const int* rp, const int* ci, const TV* v,
-                      const TX* x, TY* y, const TY* b, const TY* d, TY w, const KState* st) {
+                      const TX* x, TY* y, const TY* b, const TY* d, TY w, const KState* st,
+                      const uint8_t* fd = nullptr) {
 #define SSV_MV_CASE(L, UU)                                                                                          \
     if (lanes == L && u == UU) {                                                                                   \
-        launch_k(k_mv_spmv<TV, TX, TY, NV, L, MODE, RECIP, UU>, grid, kBlock, s, n, rp, ci, v, x, y, b, d, w, st); \
+        launch_k(k_mv_spmv<TV, TX, TY, NV, L, MODE, RECIP, UU>, grid, kBlock, s, n, rp, ci, v, x, y, b, d, w, fd, st); \
         return;                                                                                                    \
     }
     SSV_MV_CASE(2, 1)
@@ -1279,7 +1453,7 @@ static void launch_mv(int lanes, int u, int grid, cudaStream_t s, int n, const i
     SSV_MV_CASE(8, 4)
     SSV_MV_CASE(16, 4)
 #undef SSV_MV_CASE
-    launch_k(k_mv_spmv<TV, TX, TY, NV, 32, MODE, RECIP, 1>, grid, kBlock, s, n, rp, ci, v, x, y, b, d, w, st);
+    launch_k(k_mv_spmv<TV, TX, TY, NV, 32, MODE, RECIP, 1>, grid, kBlock, s, n, rp, ci, v, x, y, b, d, w, fd, st);
 }
 
 static int mv_grid(int n, int lanes, int u) {
@@ -1289,12 +1463,12 @@ static int mv_grid(int n, int lanes, int u) {
 
 template <typename TX, typename TY, int NV, int MODE, bool RECIP>
 static void launch_sell(const DevSell& S, int shape, cudaStream_t s, const TX* x, TY* y, const TY* b, const TY* d,
-                        TY w, const KState* st) {
+                        TY w, const KState* st, const uint8_t* fd = nullptr) {
     const int pairs = shape & kSellPair;  // two slices per warp
     const int per_block = (kBlock / 32) * (pairs ? 2 : 1);
     const int grid = std::max(1, (S.slices + per_block - 1) / per_block);
-#define SSV_SELL_ARGS grid, kBlock, s, S.slices, S.off.get(), S.rows.get(), S.ci.get(), S.v.get(), x, y, b, d, w, st, \
-                      S.pat_n
+#define SSV_SELL_ARGS grid, kBlock, s, S.slices, S.off.get(), S.rows.get(), S.ci.get(), S.v.get(), x, y, b, d, w, fd, \
+                      st, S.pat_n
     if constexpr (NV <= 2) {
         if (shape == (kSellDeep | 2)) {
             launch_k(k_sell_spmv_deep<TX, TY, NV, MODE, RECIP, 2>, SSV_SELL_ARGS);
@@ -1326,17 +1500,18 @@ static void launch_sell(const DevSell& S, int shape, cudaStream_t s, const TX* x
 
 template <typename TV, typename TX, typename TY, int NV, int MODE, bool RECIP>
 static void mv_spmv(const DevCsr& A, const TX* x, TY* y, const TY* b, const TY* d, TY w, const KState* st,
-                    cudaStream_t s) {
+                    cudaStream_t s, const uint8_t* fd = nullptr) {
     if constexpr (std::is_same_v<TV, double>) {
         if (A.sell_for(NV)) {
-            launch_sell<TX, TY, NV, MODE, RECIP>(A.sell, A.tuned_sell[DevCsr::nv_slot(NV)], s, x, y, b, d, w, st);
+            launch_sell<TX, TY, NV, MODE, RECIP>(A.sell, A.tuned_sell[DevCsr::nv_slot(NV)], s, x, y, b, d, w, st,
+                                                 fd);
             return;
         }
     }
     const int lanes = A.lanes_for(NV);
     const int u = A.unroll_for(NV);
     launch_mv<TV, TX, TY, NV, MODE, RECIP>(lanes, u, mv_grid(A.n, lanes, u), s, A.n, A.rp.get(), A.ci.get(),
-                                           A.val<TV>(), x, y, b, d, w, st);
+                                           A.val<TV>(), x, y, b, d, w, st, fd);
 }
 
 template <typename T, int NV, bool RECIP>
@@ -1756,40 +1931,31 @@ static void ams_cycle(AmsState& a, const double* in, double* out, const KState* 
     double* alt = a.xb.get();
     double* r = a.r.get();
     const int gm = grid_for((int64_t)n * NV, kBlock);
-    launch_k(k_mv_mask_copy<double, double, NV>, gm, kBlock, s, n, in, fd, b0, st);
+    bool fresh = a.num_smooth < 1;  // x == 0
+    if (fresh) launch_k(k_mv_mask_copy<double, double, NV>, gm, kBlock, s, n, in, fd, b0, st);
+    else launch_k(k_mv_mask_sweep<NV, RECIP>, gm, kBlock, s, n, in, fd, d, b0, cur, st);
+    int swept = fresh ? 0 : 1;  // sweeps of the first smoothing already done
+    bool written = false;       // out holds the result
     // (the fused first sweep + residual is not used on the fine level: with
     // 7.4M nonzeros its second gather, of l1, costs more than the separate
     // elementwise sweep saves)
-    bool fresh = true;      // x == 0
-    bool deferred = false;  // a lone first sweep waiting to be fused with the next residual
-    auto fine_smooth = [&]() {
-        for (int k = 0; k < a.num_smooth; ++k) {
-            if (fresh) {
-                first_sweep<double, NV, RECIP>(n, b0, d, cur, st, s);
-                fresh = false;
-            } else {
-                mv_spmv<double, double, double, NV, MV_JAC, RECIP>(a.A_bc, cur, alt, b0, d, 0.0, st, s);
-                std::swap(cur, alt);
-            }
+    // the last sweep of the cycle writes its masked result straight to out
+    auto fine_smooth = [&](bool last) {
+        for (int k = swept; k < a.num_smooth; ++k) {
+            // (not with blocks of columns, whose sweeps are short of registers)
+            const bool end = kReadAhead<NV> && last && k + 1 == a.num_smooth;
+            mv_spmv<double, double, double, NV, MV_JAC, RECIP>(a.A_bc, cur, end ? out : alt, b0, d, 0.0, st, s,
+                                                               end ? fd : nullptr);
+            if (end) written = true;
+            else std::swap(cur, alt);
         }
+        swept = 0;
     };
-    auto ensure_x = [&]() {
-        if (deferred) {
-            first_sweep<double, NV, RECIP>(n, b0, d, cur, st, s);
-            deferred = false;
-        }
+    auto residual = [&]() {  // r = b0 - A_bc x
         if (fresh) {
             SSV_CUDA(cudaMemsetAsync(cur, 0, sizeof(double) * (size_t)n * NV, s));
             fresh = false;
         }
-    };
-    auto residual = [&]() {  // r = b0 - A_bc x
-        if (deferred) {
-            first_res<double, NV, RECIP>(a.A_bc, b0, d, cur, r, st, s);
-            deferred = false;
-            return;
-        }
-        ensure_x();
         mv_spmv<double, double, double, NV, MV_RES, RECIP>(a.A_bc, cur, r, b0, nullptr, 0.0, st, s);
     };
     auto gradient = [&]() {
@@ -1814,12 +1980,11 @@ static void ams_cycle(AmsState& a, const double* in, double* out, const KState* 
         pi_prolong<TN, NV>(a, g3[0], g3[1], g3[2], cur, st, s);
     };
     if (a.cycle_type == 7) {
-        fine_smooth(); gradient(); fine_smooth(); nodal(); fine_smooth(); gradient(); fine_smooth();
+        fine_smooth(false); gradient(); fine_smooth(false); nodal(); fine_smooth(false); gradient(); fine_smooth(true);
     } else {
-        fine_smooth(); gradient(); nodal(); gradient(); fine_smooth();
+        fine_smooth(false); gradient(); nodal(); gradient(); fine_smooth(true);
     }
-    ensure_x();
-    launch_k(k_mv_mask_copy<double, double, NV>, gm, kBlock, s, n, cur, fd, out, st);
+    if (!written) launch_k(k_mv_mask_copy<double, double, NV>, gm, kBlock, s, n, cur, fd, out, st);
     SSV_LAUNCH_CHECK();
 }
 
@@ -2315,6 +2480,7 @@ static void ams_reserve(AmsState& a, int nv) {
     a.nv_alloc = nv;
     ++a.gen;  // new work buffers: graphs that captured the old ones must be rebuilt
     const double t0 = wall_seconds();
+    SSV_CUDA(cudaStreamSynchronize(stream()));  // the kernels read their matrices before their wait
     tune_lanes(a);
     a.t_tune += wall_seconds() - t0;
     {

@@ -11,9 +11,6 @@ constexpr int kBlkAhead = ST<S>::cplx ? 4 : 8;
 constexpr int kBigThreads = 256;
 constexpr int kBigWidth = 4;  // internal entries of an oversized block's row kept in registers
 
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 // One colour's run of blocks. iv holds, per slice, LANES - 1 rows of 32 couplings:
 // forward, row t the coupling to the block's row t; backward, to its row t + 1.
 template <typename S, typename SL, int LANES, bool FWD>
@@ -23,7 +20,6 @@ k_blk_sweep(int s0, int s1, const int* __restrict__ prow, const int* __restrict_
             const double* __restrict__ sc, S* y, const KState* st) {
     constexpr int A = kBlkAhead<S>;
     constexpr int NI = LANES <= 8 ? LANES - 1 : 0;  // couplings held in registers
-    pdl_trigger();
     const int sl = s0 + blockIdx.x * 4 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31, j = lane % LANES;
     const bool on = sl < s1;
@@ -51,7 +47,7 @@ k_blk_sweep(int s0, int s1, const int* __restrict__ prow, const int* __restrict_
         c[u] = u < K ? cp[u * 32] : -1;
         if (u < K) vv[u] = vp[u * 32];
     }
-    pdl_wait();
+    pdl_gate();
     if ((st && st->done) || !on) return;
     S s = ST<S>::zero(), g[A];
     if (row >= 0) {
@@ -95,7 +91,6 @@ k_big_sweep(int nlev, int nr, int width, const int* __restrict__ lev, const int*
             const int* __restrict__ xcol, const SL* __restrict__ xv, const S* __restrict__ inv,
             const S* __restrict__ x, const double* __restrict__ sc, S* y, const KState* st) {
     extern __shared__ __align__(16) unsigned char big_smem[];
-    pdl_trigger();
     const int tid = threadIdx.x;
     const int qa = lev[0];
     S* ys = reinterpret_cast<S*>(big_smem);
@@ -109,7 +104,7 @@ k_big_sweep(int nlev, int nr, int width, const int* __restrict__ lev, const int*
     }
     for (int l = tid; l <= nlev; l += kBigThreads) slev[l] = lev[l] - qa;
     if (tid == 0) ys[nr] = ST<S>::zero();
-    pdl_wait();
+    pdl_gate();
     if (st && st->done) return;
     for (int q = tid; q < nr; q += kBigThreads) {
         const int i = rows[qa + q];

@@ -18,6 +18,13 @@ constexpr int kBlock = 256;  // threads per block of the streaming kernels
 // here for its predecessor's completion and memory (griddepcontrol.wait)
 // before touching any data, then lets its own successor start launching.
 // Launched without the attribute, both instructions have no effect.
+// A kernel may read what no launch of the iteration writes (patterns,
+// coefficients) before its pdl_gate(): those reads then run behind the
+// predecessor. Only where these inputs were complete before the predecessor was
+// launched: every chain starts with a kernel that reads nothing before its gate,
+// and set-up ends with a synchronisation. (Letting the successor launch before
+// the wait as well puts several waiting kernels on the SMs at a time, whose
+// blocks then no longer spread evenly: a 357-block product 4.4 -> 6.9 us.)
 __device__ __forceinline__ void pdl_gate() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

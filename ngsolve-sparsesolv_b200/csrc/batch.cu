@@ -527,6 +527,7 @@ static void bt_pq(ssv_batch& B, cudaStream_t s) {
 // the frequencies are independent and run as parallel branches
 static void bt_precond(ssv_batch& B, const zdouble* in, zdouble* out, const KState* st, cudaStream_t s) {
     const size_t blk = (size_t)B.n * B.R;
+    PlainLaunches plain(B.branches > 1);
     B.forks.fork(s, B.branches);
     for (int f = 0; f < B.F; ++f) {
         const zdouble* i = in + f * blk;

@@ -226,6 +226,7 @@ int ssv_matrix_destroy(ssv_matrix* A) {
     return guarded([&] {
         if (!A) return;
         ssv::cocr_forget(A);
+        ssv::gmres_forget(A);
         delete A;
     });
 }

@@ -6,6 +6,9 @@
 // device; the host drives the iteration (the Gram-Schmidt of step j has j+1
 // dependent dot/update pairs) and reads two scalars per step to stop.
 #include <cmath>
+#include <map>
+#include <memory>
+#include <mutex>
 
 #include "objects.cuh"
 #include "solver_api.hpp"
@@ -20,12 +23,26 @@ __global__ void k_gm_scale(int n, double s, int zero, const S* __restrict__ x, S
         y[i] = zero ? ST<S>::zero() : ST<S>::scale(s, x[i]);
 }
 
-// w -= h v with h = H[j][i] on the device (the Gram-Schmidt update)
+// One Gram-Schmidt step in one pass over w: w -= h v with h = H[j][i] on the device, then
+// the dot product of the next basis vector with the new w (or ||w||^2 where next is null)
+// into out. Bound by launch latency at the usual sizes, so one launch a step in place of an
+// update and a dot product: GMRES(30), 59 steps on 29,667 rows, 11 to 8.8 ms with the kept
+// work vectors below.
 template <typename S>
-__global__ void k_gm_axpy(int n, const double2* __restrict__ h, const S* __restrict__ v, S* __restrict__ w) {
+__global__ void __launch_bounds__(kBlock)
+k_gm_step(int n, const double2* __restrict__ h, const S* __restrict__ v, S* __restrict__ w, const S* __restrict__ next,
+          RedBuf red, double2* out) {
     pdl_gate();
     const S hv = s_from2<S>(*h);
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) w[i] = w[i] - hv * v[i];
+    double2 part = make_double2(0.0, 0.0);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const S wi = w[i] - hv * v[i];
+        w[i] = wi;
+        if (next) part = add2(part, s_to2<S>((ST<S>::cplx ? ST<S>::conj(next[i]) : next[i]) * wi));
+        else part.x += ST<S>::norm2(wi);
+    }
+    double2 total;
+    if (grid_reduce2(part, red.partials, red.ticket, total)) *out = total;
 }
 
 template <typename S>
@@ -106,20 +123,86 @@ __global__ void k_gm_update(int n, int dim, const S* __restrict__ Z, const doubl
     }
 }
 
+// Work vectors of a solve, kept with the matrix from call to call (ten allocations and frees
+// a call cost 1 to 2 ms of a 10 ms solve, far more on a busy host; a solve whose vectors
+// exceed kGmresKeep takes 50 ms and more, and gives them back). A call takes them out of the
+// table and puts them back when it has ended well, so that a second thread on the same
+// matrix allocates its own.
+constexpr size_t kGmresKeep = size_t(64) << 20;
+
+template <typename S>
+struct GmresWork {
+    DevBuf<S> V, Z, w, r, rhs;
+    DevBuf<double2> H2, sn2, g2, yv, scal, partials;
+    DevBuf<double> cs;
+    DevBuf<unsigned int> ticket;
+    size_t bytes() const {
+        return sizeof(S) * (V.size() + Z.size() + 3 * w.size()) + sizeof(double2) * (H2.size() + 3 * sn2.size());
+    }
+};
+
+struct GmresKept {
+    std::unique_ptr<GmresWork<double>> d;
+    std::unique_ptr<GmresWork<zdouble>> z;
+};
+static std::mutex& gmres_mutex() {
+    static std::mutex m;
+    return m;
+}
+static std::map<const ssv_matrix*, GmresKept>& gmres_table() {
+    static std::map<const ssv_matrix*, GmresKept> t;
+    return t;
+}
+void gmres_forget(const ssv_matrix* A) {
+    GmresKept gone;  // freed after the lock is given up
+    std::lock_guard<std::mutex> lk(gmres_mutex());
+    auto it = gmres_table().find(A);
+    if (it == gmres_table().end()) return;
+    gone = std::move(it->second);
+    gmres_table().erase(it);
+}
+template <typename S> std::unique_ptr<GmresWork<S>>& kept_of(GmresKept& k);
+template <> std::unique_ptr<GmresWork<double>>& kept_of<double>(GmresKept& k) { return k.d; }
+template <> std::unique_ptr<GmresWork<zdouble>>& kept_of<zdouble>(GmresKept& k) { return k.z; }
+
+template <typename S>
+static std::unique_ptr<GmresWork<S>> gmres_take(const ssv_matrix* A) {
+    std::unique_ptr<GmresWork<S>> w;
+    {
+        std::lock_guard<std::mutex> lk(gmres_mutex());
+        auto it = gmres_table().find(A);
+        if (it != gmres_table().end()) w = std::move(kept_of<S>(it->second));
+    }
+    if (!w) w.reset(new GmresWork<S>());
+    return w;
+}
+template <typename S>
+static void gmres_keep(const ssv_matrix* A, std::unique_ptr<GmresWork<S>> w) {
+    if (w->bytes() > kGmresKeep) return;
+    std::lock_guard<std::mutex> lk(gmres_mutex());
+    auto& slot = kept_of<S>(gmres_table()[A]);
+    if (!slot) slot = std::move(w);
+}
+
 template <typename S>
 static void run_gmres(ssv_matrix* A, ssv_precond* pre, const uint8_t* fd, int maxiter, double tol, int restart,
                       const S* d_b, S* d_x, int* iterations) {
     cudaStream_t s = stream();
     const int n = A->rows;
-    const int g = grid_for(n, kBlock);
+    const int g = grid_vec(n);
     const S* v = reinterpret_cast<const S*>(A->val.get());
     const int m = std::max(1, std::min(maxiter, restart > 0 ? restart : maxiter));
-    DevBuf<S> V((size_t)(m + 1) * n), Z((size_t)m * n), w(n), r(n), rhs(n);
-    DevBuf<double2> H2((size_t)m * (m + 1)), sn2(m), g2(m + 1), yv(m), scal(4);
-    DevBuf<double> cs(m);
-    DevBuf<double2> partials((size_t)sm_count() * 8 + 64);
-    DevBuf<unsigned int> ticket(4);
-    SSV_CUDA(cudaMemsetAsync(ticket.get(), 0, sizeof(unsigned int) * 4, s));
+    std::unique_ptr<GmresWork<S>> work = gmres_take<S>(A);
+    GmresWork<S>& W = *work;
+    W.V.alloc((size_t)(m + 1) * n); W.Z.alloc((size_t)m * n); W.w.alloc(n); W.r.alloc(n); W.rhs.alloc(n);
+    W.H2.alloc((size_t)m * (m + 1)); W.sn2.alloc(m); W.g2.alloc(m + 1); W.yv.alloc(m); W.scal.alloc(4); W.cs.alloc(m);
+    W.partials.alloc((size_t)sm_count() * 8 + 64);
+    W.ticket.alloc(4);
+    SSV_CUDA(cudaMemsetAsync(W.ticket.get(), 0, sizeof(unsigned int) * 4, s));
+    DevBuf<S>&V = W.V, &Z = W.Z, &w = W.w, &r = W.r, &rhs = W.rhs;
+    DevBuf<double2>&H2 = W.H2, &sn2 = W.sn2, &g2 = W.g2, &yv = W.yv, &scal = W.scal, &partials = W.partials;
+    DevBuf<double>& cs = W.cs;
+    DevBuf<unsigned int>& ticket = W.ticket;
     const RedBuf red{partials.get(), ticket.get()};
     auto vcol = [&](int i) { return V.get() + (size_t)i * n; };
     auto zcol = [&](int i) { return Z.get() + (size_t)i * n; };
@@ -163,12 +246,12 @@ static void run_gmres(ssv_matrix* A, ssv_precond* pre, const uint8_t* fd, int ma
                 launch_spmv<S, S, 0>(A->lanes, n, A->rp.get(), A->ci.get(), v, zcol(j), w.get(), nullptr, fd, nullptr,
                                      RED_STORE, red, nullptr, s);
                 double2* hcol = H2.get() + (size_t)j * (m + 1);
-                for (int i = 0; i <= j; ++i) {  // modified Gram-Schmidt
-                    launch_k(k_dot<S>, g, kBlock, s, n, (const S*)vcol(i), (const S*)w.get(), conj, (KState*)nullptr,
-                             (int)RED_STORE, red, hcol + i);
-                    launch_k(k_gm_axpy<S>, g, kBlock, s, n, (const double2*)(hcol + i), (const S*)vcol(i), w.get());
-                }
-                launch_k(k_norm2<S>, g, kBlock, s, n, (const S*)w.get(), red, scal.get());
+                // modified Gram-Schmidt
+                launch_k(k_dot<S>, g, kBlock, s, n, (const S*)vcol(0), (const S*)w.get(), conj, (KState*)nullptr,
+                         (int)RED_STORE, red, hcol);
+                for (int i = 0; i <= j; ++i)
+                    launch_k(k_gm_step<S>, g, kBlock, s, n, (const double2*)(hcol + i), (const S*)vcol(i), w.get(),
+                             i < j ? (const S*)vcol(i + 1) : nullptr, red, i < j ? hcol + i + 1 : scal.get());
                 launch_k(k_gm_rotate<S>, 1, 32, s, j, m, H2.get(), cs.get(), sn2.get(), g2.get(),
                          (const double2*)scal.get(), rhs_norm, scal.get() + 1);
                 last = read2(scal.get() + 1);  // (res, h_next)
@@ -189,6 +272,7 @@ static void run_gmres(ssv_matrix* A, ssv_precond* pre, const uint8_t* fd, int ma
     SSV_LAUNCH_CHECK();
     precond_check(pre, s);
     *iterations = total;
+    gmres_keep<S>(A, std::move(work));
 }
 
 void gmres_solve_dev(ssv_matrix* A, ssv_precond* pre, const uint8_t* d_fd, int maxiter, double tol, int restart,

@@ -28,6 +28,7 @@ void gmres_solve_dev(ssv_matrix* A, ssv_precond* pre, const uint8_t* d_fd, int m
                      const void* d_b, void* d_x, int* iterations);
 void mrtr_forget(const ssv_solver* s);
 void cocr_forget(const ssv_matrix* A);
+void gmres_forget(const ssv_matrix* A);
 
 template <typename S>
 void ic_apply_dev(ssv_precond* p, const S* x, S* y, const KState* st, cudaStream_t s);

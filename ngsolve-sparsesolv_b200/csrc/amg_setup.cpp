@@ -360,7 +360,20 @@ double dense_ldlt_pseudo(const HostCsr& A, std::vector<double>& linv, std::vecto
         d[j] = zero ? 0.0 : dj;
         if (!zero) kept_min = std::min(kept_min, std::abs(dj) / diag0[j]);
         L[(size_t)j * n + j] = 1.0;
-        for (int i = j + 1; i < n; ++i) {
+        // eight rows side by side: the subtractions of one row wait for one another
+        int i = j + 1;
+        for (; i + 8 <= n; i += 8) {
+            double s[8];
+            const double* r[8];
+            for (int q = 0; q < 8; ++q) {
+                r[q] = &L[(size_t)(i + q) * n];
+                s[q] = r[q][j];
+            }
+            for (int k = 0; k < j; ++k)
+                for (int q = 0; q < 8; ++q) s[q] -= r[q][k] * w[k];
+            for (int q = 0; q < 8; ++q) L[(size_t)(i + q) * n + j] = zero ? 0.0 : s[q] / dj;
+        }
+        for (; i < n; ++i) {
             double s = L[(size_t)i * n + j];
             for (int k = 0; k < j; ++k) s -= L[(size_t)i * n + k] * w[k];
             L[(size_t)i * n + j] = zero ? 0.0 : s / dj;
@@ -371,18 +384,29 @@ double dense_ldlt_pseudo(const HostCsr& A, std::vector<double>& linv, std::vecto
     // linv row-major, linvt = its transpose (row i holds column i of L^{-1})
     linv.assign((size_t)n * n, 0.0);
     linvt.assign((size_t)n * n, 0.0);
+    // W columns at a time, side by side (a column of L^{-1} is zero above its diagonal, so
+    // its chain of subtractions starts there: -0 * L adds nothing to +0)
     auto columns = [&](int c0, int c1) {
-        std::vector<double> y(n);
-        for (int c = c0; c < c1; ++c) {
-            for (int i = 0; i < n; ++i) {
-                double s = (i == c) ? 1.0 : 0.0;
-                for (int k = 0; k < i; ++k) s -= L[(size_t)i * n + k] * y[k];
-                y[i] = s;
+        constexpr int W = 8;
+        std::vector<double> y((size_t)n * W);
+        for (int c = c0; c < c1; c += W) {
+            const int cols = std::min(W, c1 - c);
+            std::fill(y.begin(), y.end(), 0.0);
+            for (int i = c; i < n; ++i) {
+                double s[W];
+                for (int q = 0; q < W; ++q) s[q] = i == c + q ? 1.0 : 0.0;
+                for (int k = c; k < i; ++k) {
+                    const double l = L[(size_t)i * n + k];
+                    const double* yk = &y[(size_t)k * W];
+                    for (int q = 0; q < W; ++q) s[q] -= l * yk[q];
+                }
+                for (int q = 0; q < W; ++q) y[(size_t)i * W + q] = s[q];
             }
-            for (int i = 0; i < n; ++i) {
-                linv[(size_t)i * n + c] = y[i];
-                linvt[(size_t)c * n + i] = y[i];
-            }
+            for (int i = 0; i < n; ++i)
+                for (int q = 0; q < cols; ++q) {
+                    linv[(size_t)i * n + c + q] = y[(size_t)i * W + q];
+                    linvt[(size_t)(c + q) * n + i] = y[(size_t)i * W + q];
+                }
         }
     };
     const int nt = std::max(1, std::min(16, (int)std::thread::hardware_concurrency()));

@@ -102,6 +102,108 @@ constexpr bool kReadAhead = NV <= 2;
 template <typename A, typename B>
 using wider_t = std::conditional_t<(sizeof(A) >= sizeof(B)), A, B>;
 
+// Column-split rows for blocks of columns (NV = 4 or 8): G lanes share an entry and sum
+// CS = 16 bytes of its columns each, LANES / G entries of a row side by side, R of them read
+// together. An entry's x row is then gathered as one piece by neighbouring lanes instead of
+// by one lane in NV / CS loads that each touch 32 rows, the sums take CS registers instead
+// of NV, and the reduction CS shuffles a step instead of NV. A cycle of eight FP64 columns,
+// 45 k edges: 418 -> 310 us with the split of k_sell_spmv_cs and the Pi products below.
+template <typename TX, int NV>
+constexpr int kColWidth = 16 / (int)sizeof(TX);
+template <typename TX, int NV, int LANES>
+constexpr bool kColSplit = NV >= 4 && NV > kColWidth<TX, NV> && LANES * kColWidth<TX, NV> >= NV;
+
+template <int CS, typename T>
+__device__ __forceinline__ void store_row(T* __restrict__ p, const T (&o)[CS]) {
+    if constexpr (sizeof(T) == 8 && CS % 2 == 0) {
+#pragma unroll
+        for (int i = 0; i < CS / 2; ++i)
+            reinterpret_cast<double2*>(p)[i] = make_double2((double)o[2 * i], (double)o[2 * i + 1]);
+    } else if constexpr (sizeof(T) == 4 && CS % 4 == 0) {
+#pragma unroll
+        for (int i = 0; i < CS / 4; ++i)
+            reinterpret_cast<float4*>(p)[i] =
+                make_float4((float)o[4 * i], (float)o[4 * i + 1], (float)o[4 * i + 2], (float)o[4 * i + 3]);
+    } else {
+#pragma unroll
+        for (int c = 0; c < CS; ++c) p[c] = o[c];
+    }
+}
+
+template <typename TV, typename TX, typename TY, int NV, int LANES, int MODE, bool RECIP>
+__device__ __forceinline__ void
+col_split_rows(int n, const int* __restrict__ rp, const int* __restrict__ ci, const TV* __restrict__ v,
+               const TX* __restrict__ x, TY* __restrict__ y, const TY* __restrict__ b, const TY* __restrict__ d, TY w) {
+    using TA = wider_t<TV, TX>;
+    constexpr int CS = kColWidth<TX, NV>, G = NV / CS, E = LANES / G, R = 4;
+    const int sub = threadIdx.x % LANES;
+    const int c0 = (sub % G) * CS;
+    const int rpb = kBlock / LANES;
+    const int lane_row = (threadIdx.x & 31) / LANES;  // warp-uniform trip count
+    for (int row = blockIdx.x * rpb + threadIdx.x / LANES; row - lane_row < n; row += gridDim.x * rpb) {
+        const bool valid = row < n;
+        TA acc[CS];
+#pragma unroll
+        for (int c = 0; c < CS; ++c) acc[c] = TA(0);
+        const int k1 = valid ? rp[row + 1] : 0;
+        for (int k = valid ? rp[row] + sub / G : 0; k < k1; k += E * R) {
+            int j[R];
+            TA a[R];
+#pragma unroll
+            for (int u = 0; u < R; ++u) {
+                const bool on = k + u * E < k1;
+                j[u] = on ? ci[k + u * E] : -1;
+                a[u] = on ? (TA)v[k + u * E] : TA(0);
+            }
+            TX xv[R][CS];
+#pragma unroll
+            for (int u = 0; u < R; ++u)
+                if (j[u] >= 0) {
+                    if constexpr (MODE == MV_TWO)  // columns past the row count read the b slot
+                        load_row<CS>((j[u] < n ? x + (size_t)j[u] * NV
+                                               : reinterpret_cast<const TX*>(b) + (size_t)(j[u] - n) * NV) +
+                                         c0,
+                                     xv[u]);
+                    else
+                        load_row<CS>(x + (size_t)j[u] * NV + c0, xv[u]);
+                }
+#pragma unroll
+            for (int u = 0; u < R; ++u)
+                if (j[u] >= 0)
+#pragma unroll
+                    for (int c = 0; c < CS; ++c) acc[c] += a[u] * (TA)xv[u][c];
+        }
+#pragma unroll
+        for (int o = LANES / 2; o >= G; o >>= 1)
+#pragma unroll
+            for (int c = 0; c < CS; ++c) acc[c] += __shfl_down_sync(0xffffffffu, acc[c], o, LANES);
+        if (valid && sub < G) {
+            const size_t base = (size_t)row * NV + c0;
+            TY o[CS];
+            if constexpr (MODE == MV_AX || MODE == MV_TWO) {
+#pragma unroll
+                for (int c = 0; c < CS; ++c) o[c] = (TY)acc[c];
+            } else if constexpr (MODE == MV_ADD) {
+                load_row<CS>(y + base, o);
+#pragma unroll
+                for (int c = 0; c < CS; ++c) o[c] += w * (TY)acc[c];
+            } else {
+                load_row<CS>(b + base, o);
+#pragma unroll
+                for (int c = 0; c < CS; ++c) o[c] -= (TY)acc[c];
+                if constexpr (MODE == MV_JAC) {
+                    TX xo[CS];
+                    load_row<CS>(x + base, xo);
+                    const TY di = d[row];
+#pragma unroll
+                    for (int c = 0; c < CS; ++c) o[c] = RECIP ? (TY)xo[c] + o[c] * di : (TY)xo[c] + o[c] / di;
+                }
+            }
+            store_row<CS>(y + base, o);
+        }
+    }
+}
+
 // y (op)= A x with matrix values TV, input TX, output TY; accumulation in the
 // wider of TV and TX. Each LANES-wide row group handles U rows per pass of the
 // row loop and issues the loads of all U rows before using any of them, so a
@@ -113,6 +215,12 @@ __global__ void __launch_bounds__(kBlock)
 k_mv_spmv(int n, const int* __restrict__ rp, const int* __restrict__ ci, const TV* __restrict__ v,
           const TX* __restrict__ x, TY* __restrict__ y, const TY* __restrict__ b, const TY* __restrict__ d, TY w,
           const uint8_t* __restrict__ fd, const KState* st) {
+    if constexpr (U == 1 && kColSplit<TX, NV, LANES>) {
+        pdl_gate();
+        if (st && st->done) return;
+        col_split_rows<TV, TX, TY, NV, LANES, MODE, RECIP>(n, rp, ci, v, x, y, b, d, w);
+        return;
+    }
     using TA = wider_t<TV, TX>;
     const int sub = threadIdx.x % LANES;
     const int rpb = kBlock / LANES;
@@ -340,14 +448,14 @@ k_sell_spmv(int slices, const int* __restrict__ off, const int* __restrict__ row
     }
 }
 
-// Column-split form for block vectors (NV = 4 or 8): NV / 2 lanes share a
-// row and each sums two of its columns, so a warp covers 32 / (NV / 2) rows of
-// its slice per pass and walks the slice in NV / 2 passes. The x rows of a
-// step are then gathered as 64- or 32-byte pieces of few rows instead of 32
-// whole rows (a fourth of the L1 wavefronts at NV = 8, where the lane-per-row
-// form is bound by the L1/TEX pipeline); the slice's values and columns are
-// still read once. Each column is summed in its CSR column order, as in
-// k_sell_spmv.
+// Column-split form for block vectors (NV = 4 or 8): NV / 2 lanes share a row and each sums
+// two of its columns, so a warp covers 32 / (NV / 2) rows of a slice, and NV / 2 neighbouring
+// warps of a block take a slice. The x rows of a step are then gathered as 64- or 32-byte
+// pieces of few rows instead of 32 whole rows (a fourth of the L1 wavefronts at NV = 8, where
+// the lane-per-row form is bound by the L1/TEX pipeline); the slice's values and columns are
+// read once. One warp walking a slice NV / 2 times left 45 k rows with 1,400 warps on 148
+// SMs: 18.6 us a product of eight columns, 12.8 with a warp per part. Each column is summed in
+// its CSR column order, as in k_sell_spmv.
 template <typename TX, typename TY, int NV, int MODE, bool RECIP, int R>
 __global__ void __launch_bounds__(kBlock)
 k_sell_spmv_cs(int slices, const int* __restrict__ off, const int* __restrict__ rows, const int* __restrict__ ci,
@@ -363,71 +471,69 @@ k_sell_spmv_cs(int slices, const int* __restrict__ off, const int* __restrict__ 
     const int lane = threadIdx.x & 31;
     const int cg = lane % G, rl = lane / G;
     const int wpb = kBlock / 32;
-    for (int sl = blockIdx.x * wpb + threadIdx.x / 32; sl < slices; sl += gridDim.x * wpb) {
+    for (int it = blockIdx.x * wpb + threadIdx.x / 32; it < slices * G; it += gridDim.x * wpb) {
+        const int sl = it / G, ps = it % G;
         const int o0 = off[sl], e1 = off[sl + 1];
-#pragma unroll 1
-        for (int ps = 0; ps < G; ++ps) {
-            const int t = ps * RP + rl;  // this lane's row of the slice
-            const int row = rows[(size_t)sl * 32 + t];
-            int e = o0 + t;
-            TA acc[CS];
+        const int t = ps * RP + rl;  // this lane's row of the slice
+        const int row = rows[(size_t)sl * 32 + t];
+        int e = o0 + t;
+        TA acc[CS];
 #pragma unroll
-            for (int c = 0; c < CS; ++c) acc[c] = TA(0);
-            double a[R];
-            int col[R];
+        for (int c = 0; c < CS; ++c) acc[c] = TA(0);
+        double a[R];
+        int col[R];
+#pragma unroll
+        for (int u = 0; u < R; ++u) {
+            const int k = e + 32 * u;
+            a[u] = k < e1 ? v[k] : 0.0;
+            col[u] = k < e1 ? ci[k] : -1;
+        }
+        while (e < e1) {  // a slice's entry count is a multiple of 32: warp-uniform
+            double an[R];
+            int cn[R];
 #pragma unroll
             for (int u = 0; u < R; ++u) {
-                const int k = e + 32 * u;
-                a[u] = k < e1 ? v[k] : 0.0;
-                col[u] = k < e1 ? ci[k] : -1;
+                const int k = e + 32 * R + 32 * u;
+                an[u] = k < e1 ? v[k] : 0.0;
+                cn[u] = k < e1 ? ci[k] : -1;
             }
-            while (e < e1) {  // a slice's entry count is a multiple of 32: warp-uniform
-                double an[R];
-                int cn[R];
 #pragma unroll
-                for (int u = 0; u < R; ++u) {
-                    const int k = e + 32 * R + 32 * u;
-                    an[u] = k < e1 ? v[k] : 0.0;
-                    cn[u] = k < e1 ? ci[k] : -1;
+            for (int u = 0; u < R; ++u) {
+                if (col[u] >= 0) {
+                    TX xv[CS];
+                    if constexpr (MODE == MV_TWO)  // columns past the row count read the b slot
+                        load_row<CS>(col[u] < n ? x + (size_t)col[u] * NV + cg * CS
+                                                : reinterpret_cast<const TX*>(b) + (size_t)(col[u] - n) * NV +
+                                                      cg * CS,
+                                     xv);
+                    else
+                        load_row<CS>(x + (size_t)col[u] * NV + cg * CS, xv);
+#pragma unroll
+                    for (int c = 0; c < CS; ++c) acc[c] += (TA)a[u] * (TA)xv[c];
                 }
-#pragma unroll
-                for (int u = 0; u < R; ++u) {
-                    if (col[u] >= 0) {
-                        TX xv[CS];
-                        if constexpr (MODE == MV_TWO)  // columns past the row count read the b slot
-                            load_row<CS>(col[u] < n ? x + (size_t)col[u] * NV + cg * CS
-                                                    : reinterpret_cast<const TX*>(b) + (size_t)(col[u] - n) * NV +
-                                                          cg * CS,
-                                         xv);
-                        else
-                            load_row<CS>(x + (size_t)col[u] * NV + cg * CS, xv);
-#pragma unroll
-                        for (int c = 0; c < CS; ++c) acc[c] += (TA)a[u] * (TA)xv[c];
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < R; ++u) {
-                    a[u] = an[u];
-                    col[u] = cn[u];
-                }
-                e += 32 * R;
             }
-            if (row >= 0) {
-                const size_t base = (size_t)row * NV + cg * CS;
 #pragma unroll
-                for (int c = 0; c < CS; ++c) {
-                    const TY ac = (TY)acc[c];
-                    if constexpr (MODE == MV_AX || MODE == MV_TWO) {
-                        y[base + c] = ac;
-                    } else if constexpr (MODE == MV_RES) {
-                        y[base + c] = b[base + c] - ac;
-                    } else if constexpr (MODE == MV_ADD) {
-                        y[base + c] += w * ac;
-                    } else {
-                        const TY r = b[base + c] - ac;
-                        const TY xo = (TY)x[base + c];
-                        y[base + c] = RECIP ? xo + r * d[row] : xo + r / d[row];
-                    }
+            for (int u = 0; u < R; ++u) {
+                a[u] = an[u];
+                col[u] = cn[u];
+            }
+            e += 32 * R;
+        }
+        if (row >= 0) {
+            const size_t base = (size_t)row * NV + cg * CS;
+#pragma unroll
+            for (int c = 0; c < CS; ++c) {
+                const TY ac = (TY)acc[c];
+                if constexpr (MODE == MV_AX || MODE == MV_TWO) {
+                    y[base + c] = ac;
+                } else if constexpr (MODE == MV_RES) {
+                    y[base + c] = b[base + c] - ac;
+                } else if constexpr (MODE == MV_ADD) {
+                    y[base + c] += w * ac;
+                } else {
+                    const TY r = b[base + c] - ac;
+                    const TY xo = (TY)x[base + c];
+                    y[base + c] = RECIP ? xo + r * d[row] : xo + r / d[row];
                 }
             }
         }
@@ -520,6 +626,13 @@ k_sell_spmv_deep(int slices, const int* __restrict__ off, const int* __restrict_
     }
 }
 
+// Blocks of columns: G lanes share an entry of Pi and sum two columns each (as in
+// col_split_rows), SL lanes a row.
+template <int NV>
+constexpr int kPiGroups = NV >= 4 ? NV / 2 : 1;
+template <int NV, int LANES>
+constexpr int kPiLanes = LANES * kPiGroups<NV> < 32 ? LANES * kPiGroups<NV> : 32;
+
 // rx/ry/rz = Pi_{x,y,z}^T r over the shared pattern of G^T (one pass over r);
 // FP64 values and accumulation, outputs in the hierarchy type TO
 template <typename TO, int NV, int LANES>
@@ -527,10 +640,12 @@ __global__ void __launch_bounds__(kBlock)
 k_mv_pi_restrict(int n, const int* __restrict__ rp, const int* __restrict__ ci, const double* __restrict__ px,
                  const double* __restrict__ py, const double* __restrict__ pz, const double* __restrict__ r,
                  TO* __restrict__ ox, TO* __restrict__ oy, TO* __restrict__ oz, const KState* st) {
-    const int sub = threadIdx.x % LANES;
-    const int rpb = kBlock / LANES;
-    const int lane_row = (threadIdx.x & 31) / LANES;
-    int row = blockIdx.x * rpb + threadIdx.x / LANES;
+    constexpr int G = kPiGroups<NV>, W = NV / G, SL = kPiLanes<NV, LANES>, E = SL / G;
+    const int sub = threadIdx.x % SL;
+    const int c0 = (sub % G) * W;
+    const int rpb = kBlock / SL;
+    const int lane_row = (threadIdx.x & 31) / SL;
+    int row = blockIdx.x * rpb + threadIdx.x / SL;
     // entries are read one step ahead of their gathers, the first ones before the wait
     int k = 0, k1 = 0, j = -1;
     double vx = 0.0, vy = 0.0, vz = 0.0;
@@ -543,7 +658,7 @@ k_mv_pi_restrict(int n, const int* __restrict__ rp, const int* __restrict__ ci, 
         }
     };
     auto head = [&](int i) {
-        k = i < n ? rp[i] + sub : 0;
+        k = i < n ? rp[i] + sub / G : 0;
         k1 = i < n ? rp[i + 1] : 0;
         entry();
     };
@@ -558,43 +673,43 @@ k_mv_pi_restrict(int n, const int* __restrict__ rp, const int* __restrict__ ci, 
     }
     for (; row - lane_row < n; row += gridDim.x * rpb) {
         const bool valid = row < n;
-        double ax[NV], ay[NV], az[NV];
+        double ax[W], ay[W], az[W];
 #pragma unroll
-        for (int c = 0; c < NV; ++c) ax[c] = ay[c] = az[c] = 0.0;
+        for (int c = 0; c < W; ++c) ax[c] = ay[c] = az[c] = 0.0;
         while (j >= 0) {
-                double rr[NV];
-                load_row<NV>(r + (size_t)j * NV, rr);
+                double rr[W];
+                load_row<W>(r + (size_t)j * NV + c0, rr);
                 const double ux = vx, uy = vy, uz = vz;
                 if constexpr (kReadAhead<NV>) {
-                    k += LANES;
+                    k += E;
                     entry();
                 }
 #pragma unroll
-                for (int c = 0; c < NV; ++c) {
+                for (int c = 0; c < W; ++c) {
                     ax[c] += ux * rr[c];
                     ay[c] += uy * rr[c];
                     az[c] += uz * rr[c];
                 }
                 if constexpr (!kReadAhead<NV>) {
-                    k += LANES;
+                    k += E;
                     entry();
                 }
         }
         if (row + (int)gridDim.x * rpb - lane_row < n) head(row + gridDim.x * rpb);
 #pragma unroll
-        for (int o = LANES / 2; o > 0; o >>= 1)
+        for (int o = SL / 2; o >= G; o >>= 1)
 #pragma unroll
-            for (int c = 0; c < NV; ++c) {
-                ax[c] += __shfl_down_sync(0xffffffffu, ax[c], o, LANES);
-                ay[c] += __shfl_down_sync(0xffffffffu, ay[c], o, LANES);
-                az[c] += __shfl_down_sync(0xffffffffu, az[c], o, LANES);
+            for (int c = 0; c < W; ++c) {
+                ax[c] += __shfl_down_sync(0xffffffffu, ax[c], o, SL);
+                ay[c] += __shfl_down_sync(0xffffffffu, ay[c], o, SL);
+                az[c] += __shfl_down_sync(0xffffffffu, az[c], o, SL);
             }
-        if (valid && sub == 0)
+        if (valid && sub < G)
 #pragma unroll
-            for (int c = 0; c < NV; ++c) {
-                ox[(size_t)row * NV + c] = (TO)ax[c];
-                oy[(size_t)row * NV + c] = (TO)ay[c];
-                oz[(size_t)row * NV + c] = (TO)az[c];
+            for (int c = 0; c < W; ++c) {
+                ox[(size_t)row * NV + c0 + c] = (TO)ax[c];
+                oy[(size_t)row * NV + c0 + c] = (TO)ay[c];
+                oz[(size_t)row * NV + c0 + c] = (TO)az[c];
             }
     }
 }
@@ -608,10 +723,12 @@ k_mv_pi_prolong(int n, const int* __restrict__ rp, const int* __restrict__ ci, c
                 const double* __restrict__ py, const double* __restrict__ pz, const TG* __restrict__ gx,
                 const TG* __restrict__ gy, const TG* __restrict__ gz, double* __restrict__ x, double w,
                 const KState* st) {
-    const int sub = threadIdx.x % LANES;
-    const int rpb = kBlock / LANES;
-    const int lane_row = (threadIdx.x & 31) / LANES;
-    int row = blockIdx.x * rpb + threadIdx.x / LANES;
+    constexpr int G = kPiGroups<NV>, W = NV / G, SL = kPiLanes<NV, LANES>, E = SL / G;
+    const int sub = threadIdx.x % SL;
+    const int c0 = (sub % G) * W;
+    const int rpb = kBlock / SL;
+    const int lane_row = (threadIdx.x & 31) / SL;
+    int row = blockIdx.x * rpb + threadIdx.x / SL;
     int k = 0, k1 = 0, j = -1;
     double vx = 0.0, vy = 0.0, vz = 0.0;
     auto entry = [&] {
@@ -623,7 +740,7 @@ k_mv_pi_prolong(int n, const int* __restrict__ rp, const int* __restrict__ ci, c
         }
     };
     auto head = [&](int i) {
-        k = i < n ? rp[i] + sub : 0;
+        k = i < n ? rp[i] + sub / G : 0;
         k1 = i < n ? rp[i + 1] : 0;
         entry();
     };
@@ -638,47 +755,47 @@ k_mv_pi_prolong(int n, const int* __restrict__ rp, const int* __restrict__ ci, c
     }
     for (; row - lane_row < n; row += gridDim.x * rpb) {
         const bool valid = row < n;
-        double sx[NV], sy[NV], sz[NV];
+        double sx[W], sy[W], sz[W];
 #pragma unroll
-        for (int c = 0; c < NV; ++c) sx[c] = sy[c] = sz[c] = 0.0;
+        for (int c = 0; c < W; ++c) sx[c] = sy[c] = sz[c] = 0.0;
         while (j >= 0) {
-                TG vgx[NV], vgy[NV], vgz[NV];
-                load_row<NV>(gx + (size_t)j * NV, vgx);
-                load_row<NV>(gy + (size_t)j * NV, vgy);
-                load_row<NV>(gz + (size_t)j * NV, vgz);
+                TG vgx[W], vgy[W], vgz[W];
+                load_row<W>(gx + (size_t)j * NV + c0, vgx);
+                load_row<W>(gy + (size_t)j * NV + c0, vgy);
+                load_row<W>(gz + (size_t)j * NV + c0, vgz);
                 const double ux = vx, uy = vy, uz = vz;
                 if constexpr (kReadAhead<NV>) {
-                    k += LANES;
+                    k += E;
                     entry();
                 }
 #pragma unroll
-                for (int c = 0; c < NV; ++c) {
+                for (int c = 0; c < W; ++c) {
                     sx[c] += ux * (double)vgx[c];
                     sy[c] += uy * (double)vgy[c];
                     sz[c] += uz * (double)vgz[c];
                 }
                 if constexpr (!kReadAhead<NV>) {
-                    k += LANES;
+                    k += E;
                     entry();
                 }
         }
         if (row + (int)gridDim.x * rpb - lane_row < n) head(row + gridDim.x * rpb);
 #pragma unroll
-        for (int o = LANES / 2; o > 0; o >>= 1)
+        for (int o = SL / 2; o >= G; o >>= 1)
 #pragma unroll
-            for (int c = 0; c < NV; ++c) {
-                sx[c] += __shfl_down_sync(0xffffffffu, sx[c], o, LANES);
-                sy[c] += __shfl_down_sync(0xffffffffu, sy[c], o, LANES);
-                sz[c] += __shfl_down_sync(0xffffffffu, sz[c], o, LANES);
+            for (int c = 0; c < W; ++c) {
+                sx[c] += __shfl_down_sync(0xffffffffu, sx[c], o, SL);
+                sy[c] += __shfl_down_sync(0xffffffffu, sy[c], o, SL);
+                sz[c] += __shfl_down_sync(0xffffffffu, sz[c], o, SL);
             }
-        if (valid && sub == 0)
+        if (valid && sub < G)
 #pragma unroll
-            for (int c = 0; c < NV; ++c) {
-                double t = x[(size_t)row * NV + c];
+            for (int c = 0; c < W; ++c) {
+                double t = x[(size_t)row * NV + c0 + c];
                 t += w * sx[c];
                 t += w * sy[c];
                 t += w * sz[c];
-                x[(size_t)row * NV + c] = t;
+                x[(size_t)row * NV + c0 + c] = t;
             }
     }
 }
@@ -889,6 +1006,12 @@ k_mv3_spmv(Tri<T, K> t, T w, const KState* st) {
     T* __restrict__ y = t.y[q];
     const T* __restrict__ b = t.b[q];
     const T* __restrict__ d = t.d[q];
+    if constexpr (kColSplit<T, NV, LANES>) {
+        pdl_gate();
+        if (st && st->done) return;
+        col_split_rows<T, T, T, NV, LANES, MODE, RECIP>(n, rp, ci, v, x, y, b, d, w);
+        return;
+    }
     const int sub = threadIdx.x % LANES;
     const int rpb = kBlock / LANES;
     const int lane_row = (threadIdx.x & 31) / LANES;
@@ -1461,12 +1584,16 @@ static int mv_grid(int n, int lanes, int u) {
     return std::max(1, std::min((n + rpb - 1) / rpb, sm_count() * 8));
 }
 
+template <int NV>
+constexpr int kSellColGroups = NV == 4 || NV == 8 ? NV / 2 : 1;  // warps a slice takes in the column-split form
+
 template <typename TX, typename TY, int NV, int MODE, bool RECIP>
 static void launch_sell(const DevSell& S, int shape, cudaStream_t s, const TX* x, TY* y, const TY* b, const TY* d,
                         TY w, const KState* st, const uint8_t* fd = nullptr) {
     const int pairs = shape & kSellPair;  // two slices per warp
     const int per_block = (kBlock / 32) * (pairs ? 2 : 1);
-    const int grid = std::max(1, (S.slices + per_block - 1) / per_block);
+    const int items = S.slices * (shape & kSellCols ? kSellColGroups<NV> : 1);
+    const int grid = std::max(1, (items + per_block - 1) / per_block);
 #define SSV_SELL_ARGS grid, kBlock, s, S.slices, S.off.get(), S.rows.get(), S.ci.get(), S.v.get(), x, y, b, d, w, fd, \
                       st, S.pat_n
     if constexpr (NV <= 2) {
@@ -1862,7 +1989,7 @@ static void vcycle3(AmsState& a, const KState* st, cudaStream_t s, T* out[3]) {
 template <typename T, int NV, int LANES>
 static void pi_restrict_l(const AmsState& a, const double* r, T* ox, T* oy, T* oz, const KState* st,
                           cudaStream_t s) {
-    const int rpb = kBlock / LANES;
+    const int rpb = kBlock / kPiLanes<NV, LANES>;
     const int grid = std::max(1, std::min((a.Gt.n + rpb - 1) / rpb, sm_count() * 8));
     launch_k(k_mv_pi_restrict<T, NV, LANES>, grid, kBlock, s, a.Gt.n, a.Gt.rp.get(), a.Gt.ci.get(), a.Pitv[0].get(),
                                                            a.Pitv[1].get(), a.Pitv[2].get(), r, ox, oy, oz, st);
@@ -1871,7 +1998,7 @@ static void pi_restrict_l(const AmsState& a, const double* r, T* ox, T* oy, T* o
 template <typename T, int NV, int LANES>
 static void pi_prolong_l(const AmsState& a, const T* gx, const T* gy, const T* gz, double* x, const KState* st,
                          cudaStream_t s) {
-    const int rpb = kBlock / LANES;
+    const int rpb = kBlock / kPiLanes<NV, LANES>;
     const int grid = std::max(1, std::min((a.G.n + rpb - 1) / rpb, sm_count() * 8));
     launch_k(k_mv_pi_prolong<T, NV, LANES>, grid, kBlock, s, a.G.n, a.G.rp.get(), a.G.ci.get(), a.Piv[0].get(),
                                                           a.Piv[1].get(), a.Piv[2].get(), gx, gy, gz, x, a.w, st);

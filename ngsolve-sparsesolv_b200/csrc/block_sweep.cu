@@ -1,6 +1,7 @@
 // block_sweep.cu -- see block_sweep.cuh.
 #include "block_sweep.cuh"
 
+#include "host_threads.hpp"
 #include "objects.cuh"
 
 namespace ssv {
@@ -240,16 +241,22 @@ void BlockSweep<S>::build(int lanes_, const std::vector<int>& boff, const std::v
     const int slices = (int)h_prow.size() / 32;
     int smem_optin = 0;
     SSV_CUDA(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, 0));
-    int big_max = 0;
-    auto direction = [&](bool fwd, Dir& D, const std::vector<Run>& runs, const std::vector<int>& rows,
+    struct Layout {
+        std::vector<int> off, col, src, isrc, xrp, xcol, xsrc, loc, lsrc;
+        int big_max = 0;
+    } lay[2];
+    auto direction = [&](bool fwd, Dir& D, Layout& h, const std::vector<Run>& runs, const std::vector<int>& rows,
                          const std::vector<int>& lv) {
+        std::vector<int>&off = h.off, &col = h.col, &src = h.src, &isrc = h.isrc, &xrp = h.xrp, &xcol = h.xcol,
+                        &xsrc = h.xsrc, &loc = h.loc, &lsrc = h.lsrc;
         const std::vector<int>& rp = fwd ? lrp : urp;
         const std::vector<int>& ci = fwd ? lci : uci;
         // a row's off-diagonal entries and their positions in L
         auto e0 = [&](int i) { return fwd ? rp[i] : rp[i] + 1; };
         auto e1 = [&](int i) { return fwd ? rp[i + 1] - 1 : rp[i + 1]; };
         auto from = [&](int k) { return fwd ? k : usrc[k]; };
-        std::vector<int> off((size_t)slices * 2), col, src, isrc((size_t)slices * (lanes - 1) * 32, -1);
+        off.resize((size_t)slices * 2);
+        isrc.assign((size_t)slices * (lanes - 1) * 32, -1);
         std::vector<int> cnt(32);
         col.reserve(rp[n]);
         src.reserve(rp[n]);
@@ -286,7 +293,8 @@ void BlockSweep<S>::build(int lanes_, const std::vector<int>& boff, const std::v
             }
         }
         // oversized blocks
-        std::vector<int> xrp(rows.size() + 1, 0), xcol, xsrc, loc, lsrc, at(n > 0 && !rows.empty() ? n : 0, -1);
+        xrp.assign(rows.size() + 1, 0);
+        std::vector<int> at(n > 0 && !rows.empty() ? n : 0, -1);
         D.steps.clear();
         for (const Run& q : runs) {
             Step st{q.kind, q.a, q.b};
@@ -326,21 +334,27 @@ void BlockSweep<S>::build(int lanes_, const std::vector<int>& boff, const std::v
                 for (int p = qa; p < qb; ++p) at[rows[p]] = -1;
                 const size_t bytes = big_bytes<S, S>(nr, width, q.b - q.a);
                 st.smem = bytes + 1024 <= (size_t)smem_optin ? (int)bytes : 0;
-                big_max = std::max(big_max, st.smem);
+                h.big_max = std::max(h.big_max, st.smem);
             }
             D.steps.push_back(st);
         }
-        auto up = [&](DevBuf<int>& d, const std::vector<int>& h) {
-            if (h.empty()) d.release();
-            else d.upload(h.data(), h.size(), s);
-        };
-        up(D.off, off); up(D.col, col); up(D.src, src); up(D.isrc, isrc);
-        up(D.lev, lv); up(D.rows, rows); up(D.loc, loc); up(D.lsrc, lsrc);
-        up(D.xrp, xrp); up(D.xcol, xcol); up(D.xsrc, xsrc);
-        SSV_CUDA(cudaStreamSynchronize(s));
     };
-    direction(true, f, run_f, rows_f, lev_f);
-    direction(false, b, run_b, rows_b, lev_b);
+    run_threads(2, [&](int t) {  // the directions' layouts side by side
+        if (t == 0) direction(true, f, lay[0], run_f, rows_f, lev_f);
+        else direction(false, b, lay[1], run_b, rows_b, lev_b);
+    });
+    auto up = [&](DevBuf<int>& d, const std::vector<int>& h) {
+        if (h.empty()) d.release();
+        else d.upload(h.data(), h.size(), s);
+    };
+    for (int t = 0; t < 2; ++t) {
+        Dir& D = t == 0 ? f : b;
+        const Layout& h = lay[t];
+        up(D.off, h.off); up(D.col, h.col); up(D.src, h.src); up(D.isrc, h.isrc);
+        up(D.lev, t == 0 ? lev_f : lev_b); up(D.rows, t == 0 ? rows_f : rows_b);
+        up(D.loc, h.loc); up(D.lsrc, h.lsrc); up(D.xrp, h.xrp); up(D.xcol, h.xcol); up(D.xsrc, h.xsrc);
+    }
+    const int big_max = std::max(lay[0].big_max, lay[1].big_max);
     if (h_prow.empty()) prow.release();
     else prow.upload(h_prow.data(), h_prow.size(), s);
     r.alloc(h_prow.size());

@@ -84,6 +84,7 @@ void ssv_version(int* major, int* minor, int* patch) {
 const char* ssv_last_error(void) { return g_last_error.c_str(); }
 
 void ssv_set_loop_guard(int32_t max_loops) { ssv::set_loop_guard(max_loops); }
+void ssv_set_sweep_wait(int32_t tries) { ssv::set_sweep_wait(tries); }
 
 void ssv_set_alloc_budget(int64_t bytes) { ssv::alloc_budget().store(bytes < 0 ? -1 : (long long)bytes); }
 

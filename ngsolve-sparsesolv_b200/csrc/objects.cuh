@@ -201,7 +201,8 @@ void build_graph_loop_body(GraphLoop& g, cudaStream_t s, F& body, int unroll) {
 
 template <typename F>
 void build_graph_loop(GraphLoop& g, const std::string& key_in, F&& body, int unroll = 1) {
-    const std::string key = key_in + (graph_while_mode() ? "|while" : "|chunk");
+    const std::string key =
+        key_in + (graph_while_mode() ? "|while" : "|chunk") + std::to_string(sweep_wait_tries());
     if (g.exec && g.key == key) return;
     g.reset();
     cudaStream_t s = stream();

@@ -29,6 +29,10 @@ namespace ssv {
 
 struct KState;
 
+// Tries of each wait inside the sweeps before it gives up (ssv_set_sweep_wait).
+int sweep_wait_tries();
+void set_sweep_wait(int tries);
+
 // What a sweep computes, with d the row's diagonal value of fill():
 enum SweepOp : int {
     SW_DIV = 0,  // y = (x - sum) / d

@@ -208,6 +208,7 @@ SIGNATURES = [
     ("ssv_cocr_refined_solve_dev", I32, [P, P, PU8, I32, ctypes.c_double, ctypes.c_double, I32, P, P,
                                          ctypes.POINTER(ssv_refine_info)]),
     ("ssv_set_loop_guard", None, [I32]),
+    ("ssv_set_sweep_wait", None, [I32]),
     ("ssv_set_alloc_budget", None, [ctypes.c_int64]),
     ("ssv_cocr_last_launches", I32, [ctypes.POINTER(ctypes.c_int64)]),
     ("ssv_gmres_solve", I32, [P, P, PU8, I32, ctypes.c_double, I32, P, P, PI32]),

@@ -379,6 +379,7 @@ static void run_cocr_ngs(ssv_matrix* A, ssv_precond* pre, const uint8_t* fd, int
         if (left > 0) run_graph_loop(ctx.loop, dst, left);
         SSV_CUDA(cudaMemcpyAsync(&h, dst, sizeof(h), cudaMemcpyDeviceToHost, s));
         SSV_CUDA(cudaStreamSynchronize(s));
+        precond_check(pre, s);
         if (h.status == SSV_ERR_TIMEOUT) fail(SSV_ERR_TIMEOUT, "COCR loop guard fired");
         ++cycles;
         g_cocr_launches += 4 + (pre ? 0 : 1) + (int64_t)ctx.loop.body_nodes * h.loops;
@@ -413,7 +414,6 @@ static void run_cocr_ngs(ssv_matrix* A, ssv_precond* pre, const uint8_t* fd, int
         // out of iterations, or a cycle that could not take a single step
         if (used >= maxiter || h.updates == 0 || rs < 1e-300) break;
     }
-    precond_check(pre, s);
     if (refine) {
         *iterations = used;
         if (info) {
@@ -525,8 +525,8 @@ static void run_pcg(ssv_matrix* A, ssv_precond* pre, const uint8_t* fd, const ss
     if (cfg.max_iterations > 0) run_graph_loop(ctx.pcg_loop, dst, cfg.max_iterations);
     SSV_CUDA(cudaMemcpyAsync(&h, dst, sizeof(h), cudaMemcpyDeviceToHost, s));
     SSV_CUDA(cudaStreamSynchronize(s));
-    if (h.status == SSV_ERR_TIMEOUT) fail(SSV_ERR_TIMEOUT, "CG loop guard fired");
     precond_check(pre, s);
+    if (h.status == SSV_ERR_TIMEOUT) fail(SSV_ERR_TIMEOUT, "CG loop guard fired");
     std::memset(res, 0, sizeof(*res));
     res->converged = h.converged;
     res->iterations = h.iters;

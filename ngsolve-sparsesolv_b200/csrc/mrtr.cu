@@ -222,6 +222,7 @@ struct MrtrPattern {
     DevBuf<double> D, iD;
     // both sweeps in one launch each (else level by level)
     Sweep<S> sweep_f, sweep_b;
+    SweepFlag sweep_err;
     bool diag = false;  // every row has its diagonal entry
     bool swept() const { return diag && sweep_f.ready && sweep_b.ready; }
 };
@@ -294,6 +295,7 @@ void run_mrtr(ssv_solver* sv, const ssv_config& cfg, const S* d_b, S* d_x, ssv_r
         P.rows_b.upload(rws.data(), rws.size(), s);
         for (int l = 0; l < nl; ++l) P.bwd.push_back({off[l], off[l + 1]});
         if (P.diag && P.sweep_f.ready) P.sweep_b.build(n, urp, uci, false, rws, off, s);
+        P.sweep_err.init(s);
         P.Lrp.upload(lrp.data(), lrp.size(), s);
         P.Lci.upload(lci.data(), lci.size(), s);
         P.Lsrc.upload(lsrc.data(), lsrc.size(), s);
@@ -350,7 +352,7 @@ void run_mrtr(ssv_solver* sv, const ssv_config& cfg, const S* d_b, S* d_x, ssv_r
     auto forward = [&](const S* a, const S* b, S* y, KState* st) {
         if (P.swept()) {
             P.sweep_f.load(a, b, nullptr, st, s);
-            P.sweep_f.run(y, st, s);
+            P.sweep_f.run(y, st, P.sweep_err.get(), s);
             return;
         }
         for (const auto& lv : P.fwd)
@@ -360,7 +362,7 @@ void run_mrtr(ssv_solver* sv, const ssv_config& cfg, const S* d_b, S* d_x, ssv_r
     auto backward = [&](const S* a, S* y, KState* st) {
         if (P.swept()) {
             P.sweep_b.load(a, nullptr, nullptr, st, s);
-            P.sweep_b.run(y, st, s);
+            P.sweep_b.run(y, st, P.sweep_err.get(), s);
             return;
         }
         for (const auto& lv : P.bwd)
@@ -423,8 +425,8 @@ void run_mrtr(ssv_solver* sv, const ssv_config& cfg, const S* d_b, S* d_x, ssv_r
     if (!h.done) run_graph_loop(sv->loop, dst, cfg.max_iterations);
     SSV_CUDA(cudaMemcpyAsync(&h, dst, sizeof(h), cudaMemcpyDeviceToHost, s));
     SSV_CUDA(cudaStreamSynchronize(s));
+    if (P.swept()) P.sweep_err.check(s);  // the sweep before the loop
     if (h.status == SSV_ERR_TIMEOUT) fail(SSV_ERR_TIMEOUT, "SGS-MRTR loop guard fired");
-    if (P.swept()) P.sweep_f.check(s);  // the sweep before the loop
     res->converged = h.converged;
     res->iterations = h.iters;
     res->final_residual = h.final_norm / h.normalizer;

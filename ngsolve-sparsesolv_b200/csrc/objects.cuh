@@ -261,6 +261,7 @@ struct ICDevice {
     DevBuf<S> tw;  // forward-sweep output
     // both sweeps in one launch each (sweep.cuh); else level by level, or (ABMC) colour by colour
     Sweep<S> sweep_f, sweep_b;
+    SweepFlag sweep_err;
     bool swept() const { return missing_row < 0 && sweep_f.ready && sweep_b.ready; }
     // ABMC: colour by colour in the block layout (block_sweep.cuh), or by the
     // CSR factor where a block is too large for that
@@ -305,6 +306,7 @@ struct SgsDevice {
     DevBuf<S> inv, tmp;
     // both sweeps in one launch each (else level by level); values of vgen
     Sweep<S> sweep_f, sweep_b;
+    SweepFlag sweep_err;
     unsigned vgen = 0;
     bool swept() const { return sweep_f.ready && sweep_b.ready; }
 };

@@ -94,6 +94,7 @@ static void sgs_update_t(ssv_precond* p) {
     if (!g.built) {
         levels_of(n, A->h_rp, A->h_ci, false, g.fwd_lev, g.rows_f, g.sweep_f, s);
         levels_of(n, A->h_rp, A->h_ci, true, g.bwd_lev, g.rows_b, g.sweep_b, s);
+        g.sweep_err.init(s);
         g.inv.alloc(n);
         g.tmp.alloc(n);
         g.built = true;
@@ -124,8 +125,8 @@ void sgs_apply_dev(ssv_precond* p, const S* x, S* y, const KState* st, cudaStrea
         // launches below (a solve's first application runs outside its capture and refills here)
         if (!p->has_fd && g.vgen != A->vgen) sgs_fill(g, A, v, s);
         g.sweep_f.load(x, nullptr, nullptr, st, s);
-        g.sweep_f.run(g.sweep_b.xs.get(), st, s);
-        g.sweep_b.run(y, st, s);
+        g.sweep_f.run(g.sweep_b.xs.get(), st, g.sweep_err.get(), s);
+        g.sweep_b.run(y, st, g.sweep_err.get(), s);
         if (p->has_fd) launch_k(k_mask_zero<S>, grid_for(n, kBlock), kBlock, s, n, y, (const uint8_t*)p->fd.get());
         SSV_LAUNCH_CHECK();
         return;

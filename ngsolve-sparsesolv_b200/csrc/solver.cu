@@ -162,6 +162,7 @@ void ICDevice<S>::build_pattern(int n_, const std::vector<int>& rp, const std::v
     fwd_launch.clear();
     bwd_launch.clear();
     sweep_f.ready = sweep_b.ready = false;
+    sweep_err.init(s);
     std::vector<int> lrp, lci, lsrc, urp, uci, usrc;
     if (abmc) {
         // abmc_use_rcm (ic_preconditioner.hpp:97-104): the ABMC schedule is
@@ -473,7 +474,7 @@ void ICDevice<S>::apply_fwd(const S* x, const KState* st, cudaStream_t s) const 
     const double* sc = scaled_apply ? scaling.get() : nullptr;
     if (swept()) {
         sweep_f.load(x, nullptr, sc, st, s);
-        sweep_f.run(sweep_b.xs.get(), st, s);
+        sweep_f.run(sweep_b.xs.get(), st, sweep_err.get(), s);
         return;
     }
     if (blk) {
@@ -498,7 +499,7 @@ void ICDevice<S>::apply_bwd(S* y, const KState* st, cudaStream_t s) const {
     const int* uo = abmc ? uoff.get() : nullptr;
     const double* sc = scaled_apply ? scaling.get() : nullptr;
     if (swept()) {
-        sweep_b.run(y, st, s);
+        sweep_b.run(y, st, sweep_err.get(), s);
         if (sc) launch_k(k_scale_real<S>, grid_for(n, kBlock), kBlock, s, n, y, sc);
         SSV_LAUNCH_CHECK();
         return;
@@ -719,6 +720,7 @@ static void run_krylov(ssv_solver* sv, int method, const ssv_config& cfg, const 
     if (cfg.max_iterations > 0) run_graph_loop(sv->loop, dst, cfg.max_iterations);
     SSV_CUDA(cudaMemcpyAsync(&h, dst, sizeof(h), cudaMemcpyDeviceToHost, s));
     SSV_CUDA(cudaStreamSynchronize(s));
+    if (ic && ic->swept() && cfg.max_iterations <= 0) ic->sweep_err.check(s);  // the sweep without a state
     if (h.status == SSV_ERR_TIMEOUT) fail(SSV_ERR_TIMEOUT, "Krylov loop guard fired (iteration state never finished)");
     if (!h.done) fail(SSV_ERR_RUNTIME, "Krylov loop ended without a result");
 
@@ -965,16 +967,13 @@ void precond_apply_dev(ssv_precond* p, const void* d_x, void* d_y) {
     else
         precond_apply_any<zdouble>(p, static_cast<const zdouble*>(d_x), static_cast<zdouble*>(d_y), nullptr,
                                    stream());
-    SSV_CUDA(cudaStreamSynchronize(stream()));
     precond_check(p, stream());
 }
 
 void precond_check(const ssv_precond* p, cudaStream_t s) {
     auto sweeps = [&](auto& q) {
-        if (q.swept()) {
-            q.sweep_f.check(s);
-            q.sweep_b.check(s);
-        }
+        if (q.swept()) q.sweep_err.check(s);
+        else SSV_CUDA(cudaStreamSynchronize(s));
     };
     if (p && p->kind == 1) {
         if (p->A->dtype == SSV_F64) sweeps(p->ic_d);
@@ -982,6 +981,8 @@ void precond_check(const ssv_precond* p, cudaStream_t s) {
     } else if (p && p->kind == 4) {
         if (p->A->dtype == SSV_F64) sweeps(p->sgs_d);
         else sweeps(p->sgs_z);
+    } else {
+        SSV_CUDA(cudaStreamSynchronize(s));
     }
 }
 

@@ -13,8 +13,8 @@ void solver_profile(ssv_solver* sv, const char* method, const ssv_config& cfg, i
                     ssv_phase_profile* out);
 void precond_update(ssv_precond* p);
 void precond_apply_dev(ssv_precond* p, const void* d_x, void* d_y);
-// After the stream has been waited for: raises SSV_ERR_TIMEOUT if a bounded wait of the
-// preconditioner's sweeps gave up outside a solve's device state.
+// Waits for the stream; raises SSV_ERR_TIMEOUT if a bounded wait of the preconditioner's
+// sweeps gave up outside a solve's device state.
 void precond_check(const ssv_precond* p, cudaStream_t s);
 double precond_actual_shift(const ssv_precond* p);
 void matrix_spmv_dev(ssv_matrix* A, const void* d_x, void* d_y);

@@ -207,7 +207,7 @@ struct DevBuf {
         alloc(count);
         if (count) SSV_CUDA(cudaMemcpyAsync(p, h, sizeof(T) * count, cudaMemcpyHostToDevice, s));
     }
-    void zero(cudaStream_t s) {
+    void zero(cudaStream_t s) const {
         if (n) SSV_CUDA(cudaMemsetAsync(p, 0, sizeof(T) * n, s));
     }
     T* get() const { return p; }

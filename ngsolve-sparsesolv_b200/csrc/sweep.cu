@@ -292,10 +292,11 @@ k_sweep(SweepArgs a, const S* __restrict__ xs, S* out, KState* st) {
         // Every CTA has sent its last result; those on their way to a CTA that no longer waits
         // for them land before it ends.
         for (int t = 0; t < 16; ++t) __nanosleep(4096);
-        atomicExch(a.err, 1);
         if (st) {
             st->status = SSV_ERR_TIMEOUT;
             st->done = 1;
+        } else {
+            atomicExch(a.err, 1);
         }
     }
 }
@@ -414,8 +415,6 @@ bool Sweep<S>::build(int n, const std::vector<int>& rp, const std::vector<int>& 
     tx.upload(plan.tx.data(), plan.tx.size(), s);
     xs.alloc(plan.rowpos.size());
     xs.zero(s);
-    if (!err.get()) err.alloc(1);
-    err.zero(s);
     stages = 0;  // laid out by the first fill()
     SSV_CUDA(cudaStreamSynchronize(s));
     ready = true;
@@ -463,11 +462,11 @@ void Sweep<S>::load(const S* a, const S* b, const double* sc, const KState* st, 
 }
 
 template <typename S>
-void Sweep<S>::run(S* out, const KState* st, cudaStream_t s) const {
+void Sweep<S>::run(S* out, const KState* st, int* err, cudaStream_t s) const {
     int bars = 0;  // levels of the longest chunk
     for (int c = 0; c < plan.nchunks; ++c) bars = std::max(bars, plan.chunk_lev[c + 1] - plan.chunk_lev[c]);
     SweepArgs a{stream.get(), rounds.get(), round_ptr.get(), chunk_lev.get(), tx.get(), plan.nlev, plan.nchunks, bars,
-                plan.ctas, (plan.slots * (int)sizeof(S) + 127) / 128 * 128, plan.stage_bytes, stages, sweep_wait_tries(), err.get()};
+                plan.ctas, (plan.slots * (int)sizeof(S) + 127) / 128 * 128, plan.stage_bytes, stages, sweep_wait_tries(), err};
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(plan.ctas);
     cfg.blockDim = dim3(kSweepThreads);
@@ -491,14 +490,17 @@ void Sweep<S>::run(S* out, const KState* st, cudaStream_t s) const {
     });
 }
 
-template <typename S>
-void Sweep<S>::check(cudaStream_t s) const {
-    if (!ready) return;
+void SweepFlag::init(cudaStream_t s) {
+    if (!dev.get()) dev.alloc(1);
+    dev.zero(s);
+}
+
+void SweepFlag::check(cudaStream_t s) const {
     int e = 0;
-    SSV_CUDA(cudaMemcpyAsync(&e, err.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
+    SSV_CUDA(cudaMemcpyAsync(&e, dev.get(), sizeof(int), cudaMemcpyDeviceToHost, s));
     SSV_CUDA(cudaStreamSynchronize(s));
     if (!e) return;
-    SSV_CUDA(cudaMemsetAsync(err.get(), 0, sizeof(int), s));
+    dev.zero(s);
     fail(SSV_ERR_TIMEOUT, "triangular sweep: a wait gave up");
 }
 

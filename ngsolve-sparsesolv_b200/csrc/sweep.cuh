@@ -43,6 +43,15 @@ enum SweepOp : int {
 // where a row's d comes from
 enum SweepDiag : int { SD_LAST = 0, SD_FIRST = 1, SD_ARRAY = 2 };
 
+// What the sweeps of one object report that run outside a solve's state.
+struct SweepFlag {
+    DevBuf<int> dev;
+    void init(cudaStream_t s);
+    int* get() const { return dev.get(); }
+    // Waits for the stream; takes the report back and raises SSV_ERR_TIMEOUT if there is one.
+    void check(cudaStream_t s) const;
+};
+
 template <typename S>
 struct Sweep {
     SweepPlanHost plan;
@@ -51,7 +60,7 @@ struct Sweep {
     int stages = 0, smem = 0;
     bool lo = false;
     DevBuf<unsigned char> stream;
-    DevBuf<int> rowpos, pos, lev, tgt_ptr, tgt, slice_round, slice_chunk0, slice_off16, round_ptr, chunk_lev, err;
+    DevBuf<int> rowpos, pos, lev, tgt_ptr, tgt, slice_round, slice_chunk0, slice_off16, round_ptr, chunk_lev;
     DevBuf<uint8_t> cta;
     DevBuf<uint32_t> tx;
     DevBuf<SweepRound> rounds;
@@ -69,11 +78,9 @@ struct Sweep {
               bool lo_, cudaStream_t s);
     // xs[position] = sc * a - b of its row (sc, b may be null)
     void load(const S* a, const S* b, const double* sc, const KState* st, cudaStream_t s) const;
-    // Sweeps from xs into out (at the rows' output indices).
-    void run(S* out, const KState* st, cudaStream_t s) const;
-    // After the stream has been waited for: raises SSV_ERR_TIMEOUT if a bounded
-    // wait of a sweep outside a solve's state gave up.
-    void check(cudaStream_t s) const;
+    // Sweeps from xs into out (at the rows' output indices). A bounded wait that gives up
+    // is reported in st, or in err where there is no state.
+    void run(S* out, const KState* st, int* err, cudaStream_t s) const;
     int positions() const { return plan.nslices * 32; }
 };
 

@@ -42,3 +42,36 @@ def test_a_solve_whose_sweeps_give_up(no_tries, method, cplx):
     r = ss.SparseSolvSolver(A, method=method, maxiter=200).Solve(b, x)
     assert r.converged and r.iterations == r0.iterations
     assert np.abs(x - good).max() <= 1e-9 * np.abs(good).max()
+
+
+def _systems():
+    A = P.laplacian_7pt(12, 11, 13)
+    return A, P.random_rhs(A.shape[0], 0)
+
+
+def _solver(kind, A):
+    import sparsesolv_ngsolve as ss
+    if kind in ("ICCG", "SGSMRTR"):
+        s = ss.SparseSolvSolver(A, method=kind, maxiter=200)
+        return lambda b: s * b
+    pre = ss.SGSPreconditioner(A) if kind.endswith("SGS") else ss.ICPreconditioner(A)
+    if "*" not in kind:
+        return lambda b: pre * b
+    s = {"PCG": ss.PCGSolver, "COCR": ss.COCRSolver, "GMRES": ss.GMRESSolver}[kind.split("*")[0]](
+        A, pre, maxiter=200, tol=1e-10)
+    return lambda b: s * b
+
+
+@pytest.mark.parametrize("kind", ["ICCG", "SGSMRTR", "IC", "SGS", "PCG*IC", "PCG*SGS", "COCR*IC", "COCR*SGS",
+                                  "GMRES*IC", "GMRES*SGS"])
+def test_a_report_is_not_raised_by_a_later_call(no_tries, kind):
+    """The call that gave up reports it; the same handle's next calls are right and say so."""
+    A, b = _systems()
+    call = _solver(kind, A)
+    good = np.array(call(b))
+    no_tries(0)
+    with pytest.raises(RuntimeError):
+        call(b)
+    no_tries(-1)
+    for _ in range(2):
+        assert np.abs(np.array(call(b)) - good).max() <= 1e-9 * np.abs(good).max()

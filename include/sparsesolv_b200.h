@@ -139,11 +139,11 @@ const char* ssv_last_error(void);
  * max_loops > 0 sets that cap for every later solve of the process; 0
  * restores the default. */
 void ssv_set_loop_guard(int32_t max_loops);
-/* Limit of the waits inside the one-launch triangular sweeps (new: no
- * reference counterpart; a test hook for the give-up path). A wait that has
- * been tried as often as the limit says ends the sweep, and the call fails
- * with SSV_ERR_TIMEOUT. tries >= 0 sets that limit for every later launch of
- * the process (0: every wait gives up at once); < 0 restores the default. */
+/* Waits inside the one-launch triangular sweeps (new: no reference
+ * counterpart; a test hook for the give-up path). A wait that has been tried
+ * up to a fixed limit ends the sweep, and the call fails with SSV_ERR_TIMEOUT.
+ * tries = 0: in every later launch of the process each wait counts as given up
+ * from the start; any other value restores the limit. */
 void ssv_set_sweep_wait(int32_t tries);
 /* Device-allocation budget (new: no reference counterpart; a test hook for
  * the allocation-failure paths). bytes >= 0: every later device allocation of

@@ -202,7 +202,7 @@ void build_graph_loop_body(GraphLoop& g, cudaStream_t s, F& body, int unroll) {
 template <typename F>
 void build_graph_loop(GraphLoop& g, const std::string& key_in, F&& body, int unroll = 1) {
     const std::string key =
-        key_in + (graph_while_mode() ? "|while" : "|chunk") + std::to_string(sweep_wait_tries());
+        key_in + (graph_while_mode() ? "|while" : "|chunk") + (sweep_no_waits() ? "|no waits" : "");
     if (g.exec && g.key == key) return;
     g.reset();
     cudaStream_t s = stream();

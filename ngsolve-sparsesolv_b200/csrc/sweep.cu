@@ -18,9 +18,9 @@ constexpr int kAhead = 4;
 constexpr int kBarBytes = (2 * kMaxStages + kSweepMaxLevels + 2) * 8;
 // tries of a wait before it gives up (a try suspends for up to a microsecond or so)
 constexpr int kWaitTries = 1 << 18;
-static std::atomic<int> g_wait_tries{kWaitTries};
-int sweep_wait_tries() { return g_wait_tries; }
-void set_sweep_wait(int tries) { g_wait_tries = tries < 0 ? kWaitTries : tries; }
+static std::atomic<bool> g_no_waits{false};
+bool sweep_no_waits() { return g_no_waits; }
+void set_sweep_wait(int tries) { g_no_waits = tries == 0; }
 
 struct SweepArgs {
     const unsigned char* stream;
@@ -28,7 +28,7 @@ struct SweepArgs {
     const int* round_ptr;
     const int* chunk_lev;
     const uint32_t* tx;
-    int nlev, nchunks, bars, ctas, win_bytes, stage_bytes, stages, tries;
+    int nlev, nchunks, bars, ctas, win_bytes, stage_bytes, stages, no_waits;
     int* err;
 };
 
@@ -58,7 +58,8 @@ __device__ __forceinline__ void bar_arrive_cluster(unsigned b) {
 __device__ __forceinline__ void bar_arrive(unsigned b) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(b) : "memory");
 }
-// Waits for the phase of the given parity; false after `tries`. CLUSTER: what other CTAs
+// Waits for the phase of the given parity; false after kWaitTries (a constant: a limit in a
+// register costs the sweep 5 %). CLUSTER: what other CTAs
 // wrote to global memory before they arrived is visible too.
 template <bool CLUSTER = false>
 __device__ __forceinline__ bool bar_try(unsigned b, unsigned parity) {
@@ -80,8 +81,8 @@ __device__ __forceinline__ bool bar_try(unsigned b, unsigned parity) {
     return ok != 0;
 }
 template <bool CLUSTER = false>
-__device__ __forceinline__ bool bar_wait(unsigned b, unsigned parity, int tries) {
-    for (int t = 0; t < tries; ++t)
+__device__ __forceinline__ bool bar_wait(unsigned b, unsigned parity) {
+    for (int t = 0; t < kWaitTries; ++t)
         if (bar_try<CLUSTER>(b, parity)) return true;
     return false;
 }
@@ -138,7 +139,7 @@ k_sweep(SweepArgs a, const S* __restrict__ xs, S* out, KState* st) {
     // a finished solve: no round is issued or waited for (the whole cluster reads the same state)
     const bool idle = st && st->done;
     // A wait that gives up ends this warp's part; the others' waits on it then give up too.
-    bool bad = false;
+    bool bad = a.no_waits != 0;
     if (warp == kComputeWarps) {  // producer: streams the rounds
         int issued = 0;
         int sg = 0;
@@ -152,7 +153,7 @@ k_sweep(SweepArgs a, const S* __restrict__ xs, S* out, KState* st) {
             for (int q = q0; q < min(q0 + 32, nr); ++q) {
                 const unsigned off = __shfl_sync(0xffffffffu, d.x, q - q0), bytes = __shfl_sync(0xffffffffu, d.y, q - q0);
                 const unsigned pos = __shfl_sync(0xffffffffu, d.z, q - q0), nsl = __shfl_sync(0xffffffffu, d.w, q - q0);
-                if (q >= a.stages) bad = __any_sync(0xffffffffu, !bar_wait(empty + 8 * sg, turn, a.tries));
+                if (q >= a.stages) bad = __any_sync(0xffffffffu, !bar_wait(empty + 8 * sg, turn));
                 if (bad) break;
                 if (lane == 0) {
                     const unsigned xb = nsl * 32 * (unsigned)sizeof(S);
@@ -169,15 +170,14 @@ k_sweep(SweepArgs a, const S* __restrict__ xs, S* out, KState* st) {
                 }
             }
         }
-        // every copy has landed before the CTA ends (whatever limit the other waits have)
-        for (int q = max(0, issued - a.stages); q < issued; ++q)
-            bar_wait(full + 8 * (q % a.stages), (q / a.stages) & 1, kWaitTries);
+        // every copy has landed before the CTA ends
+        for (int q = max(0, issued - a.stages); q < issued; ++q) bar_wait(full + 8 * (q % a.stages), (q / a.stages) & 1);
     } else {
         int chunk = 0, waited = 0;  // levels of the chunk whose values have arrived
         auto meet = [&] {  // the computing warps of all CTAs
             __syncwarp();
             if (lane < a.ctas) bar_arrive_cluster(peer_addr(cbar, lane));
-            bad = __any_sync(0xffffffffu, bad || !bar_wait<true>(cbar, chunk & 1, a.tries));
+            bad = __any_sync(0xffffffffu, bad || !bar_wait<true>(cbar, chunk & 1));
         };
         // The groups take the rounds in turn: while one finishes a level, the next ones have
         // their records and early entries behind them.
@@ -185,14 +185,13 @@ k_sweep(SweepArgs a, const S* __restrict__ xs, S* out, KState* st) {
         int sg = grp % a.stages;
         unsigned turn = (grp / a.stages) & 1;
         for (int q = grp; q < nr && !idle; q += kSweepGroups) {
-            bad = __any_sync(0xffffffffu, bad || !bar_wait(full + 8 * sg, turn, a.tries));
+            bad = __any_sync(0xffffffffu, bad || !bar_wait(full + 8 * sg, turn));
             if (bad) break;
             const unsigned char* stage = ring + (size_t)sg * a.stage_bytes;
             const SweepRound h = *reinterpret_cast<const SweepRound*>(stage);
-            // levels whose results have arrived (a wait that gave up is agreed on by the warp
-            // below; the levels after it are not waited for, each up to the limit again)
+            // levels whose results have arrived (a wait that gave up is agreed on by the warp below)
             auto wait_levels = [&](int upto) {
-                for (; waited < upto && !bad; ++waited) bad = !bar_wait(lbar + 8 * waited, chunk & 1, a.tries);
+                for (; waited < upto; ++waited) bad |= !bar_wait(lbar + 8 * waited, chunk & 1);
             };
             for (; chunk < h.chunk; ++chunk) {
                 meet();
@@ -466,7 +465,7 @@ void Sweep<S>::run(S* out, const KState* st, int* err, cudaStream_t s) const {
     int bars = 0;  // levels of the longest chunk
     for (int c = 0; c < plan.nchunks; ++c) bars = std::max(bars, plan.chunk_lev[c + 1] - plan.chunk_lev[c]);
     SweepArgs a{stream.get(), rounds.get(), round_ptr.get(), chunk_lev.get(), tx.get(), plan.nlev, plan.nchunks, bars,
-                plan.ctas, (plan.slots * (int)sizeof(S) + 127) / 128 * 128, plan.stage_bytes, stages, sweep_wait_tries(), err};
+                plan.ctas, (plan.slots * (int)sizeof(S) + 127) / 128 * 128, plan.stage_bytes, stages, sweep_no_waits(), err};
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(plan.ctas);
     cfg.blockDim = dim3(kSweepThreads);

@@ -29,8 +29,8 @@ namespace ssv {
 
 struct KState;
 
-// Tries of each wait inside the sweeps before it gives up (ssv_set_sweep_wait).
-int sweep_wait_tries();
+// Whether every wait inside the sweeps gives up at once (ssv_set_sweep_wait).
+bool sweep_no_waits();
 void set_sweep_wait(int tries);
 
 // What a sweep computes, with d the row's diagonal value of fill():

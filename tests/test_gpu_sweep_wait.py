@@ -1,8 +1,7 @@
 """The give-up path of the one-launch triangular sweeps (csrc/sweep.cu). Every
-wait inside them is bounded; with a limit of no tries at all
-(ssv_set_sweep_wait(0)) each warp gives up at its first wait, the copies in
-flight land, the kernel ends and the call returns SSV_ERR_TIMEOUT. Nothing
-hangs, and the context and the handles stay usable."""
+wait inside them is bounded; after ssv_set_sweep_wait(0) each warp counts its
+waits as given up from the start, the kernel ends and the call returns
+SSV_ERR_TIMEOUT. Nothing hangs, and the context and the handles stay usable."""
 from __future__ import annotations
 
 import numpy as np

@@ -321,21 +321,19 @@ void ICDevice<S>::build_pattern(int n_, const std::vector<int>& rp, const std::v
         };
         for (int c = 0; c < num_colors; ++c) add_colour(c, true);
         for (int c = num_colors - 1; c >= 0; --c) add_colour(c, false);
-        // Colours of few rows: the factor's own level sets through the one-launch sweeps. A level
-        // takes 0.6 us there while it fills the cluster at most (about 1024 real rows), more in
-        // proportion beyond; a colour's launch takes 2.6 us. Measured forward / backward: 24x25x23
-        // (25 levels of 552 rows, 9 launches) 14.9 / 13.7 against 23.8 / 20.7 us; 64^3 (47 levels
-        // of 5577, 10 launches) 116 / 123 against 38 / 33 us.
+        // Colours of few rows: the factor's own level sets through the one-launch sweeps, where
+        // these are estimated to take less than the launches of the colours, 2.4 us each (1.8 to
+        // 3.2 measured). Forward / backward, sweeps against launches: 24^3 14.4 / 13.1 against
+        // 21.3 / 18.9 us, 41^3 29.1 / 25.8 against 27.2 / 23.8, 64^3 116 / 122 against 36 / 30;
+        // complex, 12^3 18.3 / 16.5 against 20.6 / 17.0, 16^3 25.4 / 23.2 against 21.2 / 17.7.
+        const double launches = 2.4 * (double)run_f.size();
+        std::vector<int> rws, off;
         const int nl = build_levels(n, lrp.data(), lci.data(), false, lev);
-        const double fill = std::max(1.0, (double)n / std::max(nl, 1) * (ST<S>::cplx ? 2 : 1) / 1024.0);
-        if (0.6 * nl * fill < 2.6 * (double)run_f.size()) {
-            std::vector<int> rws, off;
-            group_by_level(lev, nl, rws, off);
-            if (sweep_f.build(n, lrp, lci, true, rws, off, s)) {
-                const int nu = build_levels(n, urp.data(), uci.data(), true, lev);
-                group_by_level(lev, nu, rws, off);
-                sweep_b.build(n, urp, uci, false, rws, off, s);
-            }
+        group_by_level(lev, nl, rws, off);
+        if (sweep_f.build(n, lrp, lci, true, rws, off, launches, s)) {
+            const int nu = build_levels(n, urp.data(), uci.data(), true, lev);
+            group_by_level(lev, nu, rws, off);
+            sweep_b.build(n, urp, uci, false, rws, off, launches, s);
         }
         if (!swept())
             blocks.build(lanes_blk, bo, run_f, run_b, h_rows_f, h_lev_f, h_rows_b, h_lev_b, lrp, lci, urp, uci, usrc, s);

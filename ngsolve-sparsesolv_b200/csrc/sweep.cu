@@ -395,12 +395,14 @@ static void sweep_kernel(bool lo, F&& f) {
 
 template <typename S>
 bool Sweep<S>::build(int n, const std::vector<int>& rp, const std::vector<int>& ci, bool fwd_,
-                     const std::vector<int>& rows, const std::vector<int>& off, cudaStream_t s) {
+                     const std::vector<int>& rows, const std::vector<int>& off, double worth, cudaStream_t s) {
     ready = false;
     fwd = fwd_;
     if (!plan.build(n, rp.data(), ci.data(), fwd, rows, off, (int)sizeof(S), kSmemBytes - kBarBytes, kStageBytes,
-                    kSweepMaxCtas))
+                    kSweepMaxCtas, worth)) {
+        plan = SweepPlanHost();
         return false;
+    }
     rowpos.upload(plan.rowpos.data(), plan.rowpos.size(), s);
     pos.upload(plan.pos.data(), plan.pos.size(), s);
     lev.upload(plan.lev.data(), plan.lev.size(), s);

@@ -67,10 +67,15 @@ struct Sweep {
     DevBuf<S> xs;  // inputs by position
 
     // Plans the sweep for a triangular part of the pattern (entries j < i or
-    // j > i of every row); false (and ready = false) where it does not fit --
-    // the caller then launches level by level.
-    bool build(int n, const std::vector<int>& rp, const std::vector<int>& ci, bool fwd,
-               const std::vector<int>& rows, const std::vector<int>& off, cudaStream_t s);
+    // j > i of every row); false (and ready = false) where it does not fit or is
+    // estimated to take more than `worth` us, the time of the caller's other way.
+    bool build(int n, const std::vector<int>& rp, const std::vector<int>& ci, bool fwd, const std::vector<int>& rows,
+               const std::vector<int>& off, double worth, cudaStream_t s);
+    // The same against a launch per level.
+    bool build(int n, const std::vector<int>& rp, const std::vector<int>& ci, bool fwd, const std::vector<int>& rows,
+               const std::vector<int>& off, cudaStream_t s) {
+        return build(n, rp, ci, fwd, rows, off, level_launches_us(n, rp.data(), rows, off, (int)sizeof(S)), s);
+    }
     // Writes the records from the CSR values: d from the row's last or first
     // entry or from darr; omap = output index of every row (null = the row).
     // lo_ stores the coefficients in the FP32 form.

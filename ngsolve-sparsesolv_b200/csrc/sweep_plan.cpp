@@ -17,13 +17,57 @@ static int pick_ctas(int n, int nlev, int ctas_max) {
     return std::min(c, ctas_max);
 }
 
+// What a sweep takes, in us. A level takes what its busiest CTA takes for its rounds: so much
+// a round, a slice, an entry and a target of the padded rows, and an entry of an earlier level
+// in a chunk after the first (read one by one); changing to another chunk and starting the
+// sweep come on top. Fitted to 150 real and 110 complex sweeps of 5 to 1400 us (grids of 12^3
+// to 160^3 rows in natural, random and coloured order, edge matrices, scattered and layered
+// patterns), which it meets to 7 and 14 % (standard deviation).
+struct SweepCost {
+    double round, slice, entry, target, far, chunk;
+};
+constexpr SweepCost kCostReal{0.264, 0.0, 0.005, 0.039, 0.033, 10.2};
+constexpr SweepCost kCostComplex{0.384, 0.154, 0.016, 0.098, 0.063, 1.9};
+constexpr double kCostStart = 3.9;  // 4.8 with the load of the inputs (forward), 3.0 without
+
+// A launch takes 2.3 us on a few short rows. A thread walks its row alone (0.08 us an entry of
+// the longest row), and rows that do not follow one another are read in pieces: longer by the
+// entry and by the row, and by up to 1.7 us where the factor and the vectors no longer stay in
+// L2. Within 13 % of 260 measured sweeps of 2 to 7000 us, which fails only where no cluster
+// competes (coloured levels of 100,000 rows and more, twice the estimate).
+double level_launches_us(int n, const int* rp, const std::vector<int>& rows, const std::vector<int>& off, int sbytes) {
+    const double bytes = (double)rp[n] * (4 + sbytes) + (double)n * (8 + 3 * sbytes);
+    const double miss = std::min(1.0, std::max(0.0, (bytes - 40e6) / 60e6));
+    double us = 0.0;
+    for (size_t l = 0; l + 1 < off.size(); ++l) {
+        int longest = 0, pieces = 0;
+        for (int q = off[l]; q < off[l + 1]; ++q) {
+            longest = std::max(longest, rp[rows[q] + 1] - rp[rows[q]]);
+            pieces += q == off[l] || rows[q] != rows[q - 1] + 1;
+        }
+        const int w = off[l + 1] - off[l];
+        if (w <= 0) continue;
+        const double apart = (double)pieces / w;
+        us += 2.27 + (0.08 + 0.10 * apart) * longest * (sbytes > 8 ? 1.6 : 1.0) + apart * (36e-6 * w + 1.7 * miss);
+    }
+    return us;
+}
+
 bool SweepPlanHost::build(int n_, const int* rp, const int* ci, bool fwd, const std::vector<int>& rows,
-                          const std::vector<int>& off, int sbytes_, int smem, int stage, int ctas_max) {
+                          const std::vector<int>& off, int sbytes_, int smem, int stage, int ctas_max, double worth) {
     n = n_;
     nlev = (int)off.size() - 1;
     sbytes = sbytes_;
     if (n <= 0 || nlev <= 0) return false;
     ctas = pick_ctas(n, nlev, std::min(ctas_max, kSweepMaxCtas));
+    const SweepCost& cost = sbytes > 8 ? kCostComplex : kCostReal;
+    // the least it can take, from the widths alone: wide levels need no plan to be refused
+    us = kCostStart;
+    for (int l = 0; l < nlev; ++l) {
+        const int sl = ((off[l + 1] - off[l] + 31) / 32 + ctas - 1) / ctas;
+        us += cost.round * ((sl + kSweepWarps - 1) / kSweepWarps) + cost.slice * sl;
+    }
+    if (us > worth) return false;
     // positions, owners, levels
     rowpos.clear();
     rowpos.reserve((size_t)n + (size_t)nlev * 16 + 64);
@@ -93,7 +137,7 @@ bool SweepPlanHost::build(int n_, const int* rp, const int* ci, bool fwd, const 
     }
     chunk_lev.push_back(nlev);
     nchunks = (int)chunk_lev.size() - 1;
-    // targets inside the chunk, and the bytes each level sends where
+    // the chunk of each level; owners with a dependent row inside the chunk
     std::vector<int> lev_chunk(nlev);
     for (int c = 0; c < nchunks; ++c)
         for (int l = chunk_lev[c]; l < chunk_lev[c + 1]; ++l) lev_chunk[l] = c;
@@ -105,24 +149,8 @@ bool SweepPlanHost::build(int n_, const int* rp, const int* ci, bool fwd, const 
                 if ((fwd ? j < i : j > i) && lev_chunk[lev[j]] == lev_chunk[lev[i]]) need[j] |= 1u << cta[i];
             }
     }
-    tgt_ptr.assign(n + 1, 0);
-    for (int i = 0; i < n; ++i) tgt_ptr[i + 1] = tgt_ptr[i] + __builtin_popcount(need[i]);
-    tgt.resize(tgt_ptr[n]);
-    tx.assign((size_t)nlev * ctas, 0u);
     std::vector<int> nt(nslices, 0);
-    for (int l = 0; l < nlev; ++l) {
-        if (l == chunk_lev[lev_chunk[l]]) std::fill(used.begin(), used.end(), 1);
-        for (int q = off[l]; q < off[l + 1]; ++q) {
-            const int i = rows[q];
-            int k = tgt_ptr[i];
-            for (uint32_t m = need[i]; m; m &= m - 1) {
-                const int c = __builtin_ctz(m);
-                tgt[k++] = c << 24 | used[c]++;
-                tx[(size_t)l * ctas + c] += (uint32_t)sbytes;
-            }
-            nt[pos[i] / 32] = std::max(nt[pos[i] / 32], k - tgt_ptr[i]);
-        }
-    }
+    for (int i = 0; i < n; ++i) nt[pos[i] / 32] = std::max(nt[pos[i] / 32], __builtin_popcount(need[i]));
     // rounds: slices of one CTA and level, as many as the warps and a stage take
     std::vector<std::vector<SweepRound>> rc(ctas);
     slice_round.assign(nslices, 0);
@@ -157,6 +185,37 @@ bool SweepPlanHost::build(int n_, const int* rp, const int* ci, bool fwd, const 
             q.chunk = lev_chunk[l];
             rc[c].push_back(q);
             slice_round[s] = (int)rc[c].size() - 1;
+        }
+    }
+    // what these rounds take, level by level
+    std::vector<double> level(nlev, 0.0), part(nlev);
+    for (int c = 0; c < ctas; ++c) {
+        std::fill(part.begin(), part.end(), 0.0);
+        for (const SweepRound& r : rc[c]) {
+            const int ke = r.ke_kl & 0xffff;
+            part[chunk_lev[r.chunk] + r.lev] += cost.round + cost.slice * r.nsl + cost.entry * (ke + (r.ke_kl >> 16)) +
+                                                cost.target * r.nt + cost.far * (r.chunk > 0 ? ke : 0);
+        }
+        for (int l = 0; l < nlev; ++l) level[l] = std::max(level[l], part[l]);
+    }
+    us = kCostStart + cost.chunk * (nchunks - 1);
+    for (double l : level) us += l;
+    if (us > worth) return false;
+    // targets inside the chunk, and the bytes each level sends where
+    tgt_ptr.assign(n + 1, 0);
+    for (int i = 0; i < n; ++i) tgt_ptr[i + 1] = tgt_ptr[i] + __builtin_popcount(need[i]);
+    tgt.resize(tgt_ptr[n]);
+    tx.assign((size_t)nlev * ctas, 0u);
+    for (int l = 0; l < nlev; ++l) {
+        if (l == chunk_lev[lev_chunk[l]]) std::fill(used.begin(), used.end(), 1);
+        for (int q = off[l]; q < off[l + 1]; ++q) {
+            const int i = rows[q];
+            int k = tgt_ptr[i];
+            for (uint32_t m = need[i]; m; m &= m - 1) {
+                const int c = __builtin_ctz(m);
+                tgt[k++] = c << 24 | used[c]++;
+                tx[(size_t)l * ctas + c] += (uint32_t)sbytes;
+            }
         }
     }
     round_ptr.assign(ctas + 1, 0);

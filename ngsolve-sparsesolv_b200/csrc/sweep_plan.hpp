@@ -53,13 +53,16 @@ struct SweepPlanHost {
     std::vector<int> round_ptr;      // ctas + 1
     std::vector<int> chunk_lev;      // nchunks + 1: first level of each chunk
     std::vector<uint32_t> tx;        // level * ctas + cta: bytes the level sends to that CTA
+    double us = 0.0;      // estimated time of the sweep
 
     // Plans the sweep over the entries j < i (fwd) or j > i of the CSR pattern,
     // rows grouped by level (rows, off). `smem` = bytes for the window and
     // kSweepMinStages rounds, `stage` = most bytes of a round, ctas_max = largest
-    // cluster. False where a level does not fit the windows or a row a round.
+    // cluster. False where a level does not fit the windows or a row a round, or where
+    // the sweep is estimated to take more than `worth` us, the time of the other way: at
+    // most 16 of the SMs work, so wide levels are better launched one by one.
     bool build(int n, const int* rp, const int* ci, bool fwd, const std::vector<int>& rows,
-               const std::vector<int>& off, int sbytes, int smem, int stage, int ctas_max);
+               const std::vector<int>& off, int sbytes, int smem, int stage, int ctas_max, double worth = 1e300);
     // Stream offsets for coefficients of vbytes each.
     void layout(int vbytes);
     // a row's record: input scale, K coefficients, K columns, output index, targets
@@ -72,5 +75,8 @@ struct SweepPlanHost {
         return -1;
     }
 };
+
+// Estimated time in us of the same sweep with a launch per level, a thread per row.
+double level_launches_us(int n, const int* rp, const std::vector<int>& rows, const std::vector<int>& off, int sbytes);
 
 }  // namespace ssv

@@ -10,7 +10,7 @@ namespace ssv {
 // kStageBytes each, the window of results the rest
 constexpr int kSmemBytes = 220 * 1024;
 constexpr int kStageBytes = 40 * 1024;
-constexpr int kMaxStages = 8;
+constexpr int kMaxStages = kSweepMaxStages;
 constexpr int kComputeWarps = kSweepWarps * kSweepGroups;
 constexpr int kSweepThreads = (kComputeWarps + 1) * 32;
 // late entries and targets of a row that are in registers before its level is due
@@ -434,7 +434,7 @@ void Sweep<S>::fill(SweepOp op, const int* rp, const int* ci, const S* v, int dm
         rounds.upload(plan.rounds.data(), plan.rounds.size(), s);
         slice_off16.upload(plan.slice_off16.data(), plan.slice_off16.size(), s);
         const int wb = (plan.slots * (int)sizeof(S) + 127) / 128 * 128;
-        const int st = std::min(kMaxStages, (kSmemBytes - wb - kBarBytes) / plan.stage_bytes);
+        const int st = plan.ring_stages(kSmemBytes - wb - kBarBytes);
         smem = wb + st * plan.stage_bytes + kBarBytes;
         sweep_kernel<S>(lo, [&](auto k) {
             SSV_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));

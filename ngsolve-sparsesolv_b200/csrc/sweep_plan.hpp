@@ -3,6 +3,7 @@
 // rounds each CTA streams through, and where each result is needed.
 #pragma once
 
+#include <algorithm>
 #include <cstddef>
 #include <cstdint>
 #include <vector>
@@ -11,9 +12,14 @@ namespace ssv {
 
 constexpr int kSweepWarps = 4;        // computing warps of a group: slices of 32 rows in a round
 constexpr int kSweepGroups = 4;       // groups of a CTA, which take its rounds in turn
-// stages of a CTA's ring at least: every group must be able to hold its next round, or a
-// group that waits for the others between chunks waits for ever
+// Stages of a CTA's ring: at least one for each group's next round, or a group that waits for
+// the others between chunks waits for ever; and a whole multiple of the groups, so that each
+// stage belongs to one group. A warp then has waited for every phase of its stages' barriers.
+// On a stage that another group used last, it could come while that group's copy is still under
+// way, take the phase before it, which has the parity it waits for, for its own, and work on
+// what lies there.
 constexpr int kSweepMinStages = kSweepGroups;
+constexpr int kSweepMaxStages = 2 * kSweepGroups;
 constexpr int kSweepMaxLevels = 512;  // levels of a chunk (one mbarrier each)
 constexpr int kSweepMaxCtas = 16;
 constexpr int kSweepHeader = 32;      // bytes in front of a round's records
@@ -65,6 +71,10 @@ struct SweepPlanHost {
                const std::vector<int>& off, int sbytes, int smem, int stage, int ctas_max, double worth = 1e300);
     // Stream offsets for coefficients of vbytes each.
     void layout(int vbytes);
+    // stages of a ring in that many bytes
+    int ring_stages(int bytes) const {
+        return std::min(kSweepMaxStages, bytes / stage_bytes / kSweepGroups * kSweepGroups);
+    }
     // a row's record: input scale, K coefficients, K columns, output index, targets
     static constexpr int row_bytes(int K, int nt, int vbytes, int sbytes) {
         return sbytes + K * (vbytes + 4) + 4 + 4 * nt;

@@ -28,7 +28,7 @@ struct SweepArgs {
     const int* round_ptr;
     const int* chunk_lev;
     const uint32_t* tx;
-    int nlev, nchunks, bars, ctas, win_bytes, stage_bytes, stages, no_waits;
+    int nchunks, bars, ctas, win_bytes, stage_bytes, stages, no_waits;
     int* err;
 };
 
@@ -394,12 +394,54 @@ static void sweep_kernel(bool lo, F&& f) {
 }
 
 template <typename S>
+static void allow_clusters(bool lo) {
+    sweep_kernel<S>(lo, [](auto k) {
+        SSV_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
+        SSV_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    });
+}
+
+// Most CTAs of a cluster that the device can place with all the shared memory they may take:
+// 16 on a whole B200, fewer (or none: 0) on a partition of one. Asked once for each device.
+template <typename S>
+static int placeable_ctas() {
+    constexpr int kDevices = 64;
+    static std::atomic<int> known[kDevices];  // ctas + 1
+    int dev = 0;
+    SSV_CUDA(cudaGetDevice(&dev));
+    if (dev < kDevices && known[dev] > 0) return known[dev] - 1;
+    int ctas = kSweepMaxCtas;
+    for (bool lo : {false, true}) {
+        allow_clusters<S>(lo);
+        sweep_kernel<S>(lo, [&](auto k) {
+            for (; ctas > 0; ctas /= 2) {
+                cudaLaunchAttribute at[1];
+                at[0].id = cudaLaunchAttributeClusterDimension;
+                at[0].val.clusterDim.x = ctas;
+                at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+                cudaLaunchConfig_t cfg = {};
+                cfg.gridDim = dim3(ctas);
+                cfg.blockDim = dim3(kSweepThreads);
+                cfg.dynamicSmemBytes = kSmemBytes;
+                cfg.attrs = at;
+                cfg.numAttrs = 1;
+                int clusters = 0;
+                if (cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) == cudaSuccess && clusters > 0) break;
+                cudaGetLastError();
+            }
+        });
+    }
+    if (dev < kDevices) known[dev] = ctas + 1;
+    return ctas;
+}
+
+template <typename S>
 bool Sweep<S>::build(int n, const std::vector<int>& rp, const std::vector<int>& ci, bool fwd_,
                      const std::vector<int>& rows, const std::vector<int>& off, double worth, cudaStream_t s) {
     ready = false;
     fwd = fwd_;
     if (!plan.build(n, rp.data(), ci.data(), fwd, rows, off, (int)sizeof(S), kSmemBytes - kBarBytes, kStageBytes,
-                    kSweepMaxCtas, worth)) {
+                    placeable_ctas<S>(), worth)) {
         plan = SweepPlanHost();
         return false;
     }
@@ -436,10 +478,7 @@ void Sweep<S>::fill(SweepOp op, const int* rp, const int* ci, const S* v, int dm
         const int wb = (plan.slots * (int)sizeof(S) + 127) / 128 * 128;
         const int st = plan.ring_stages(kSmemBytes - wb - kBarBytes);
         smem = wb + st * plan.stage_bytes + kBarBytes;
-        sweep_kernel<S>(lo, [&](auto k) {
-            SSV_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-            SSV_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        });
+        allow_clusters<S>(lo);
         const int nq = (int)plan.rounds.size();
         k_sweep_heads<<<(nq + 255) / 256, 256, 0, s>>>(nq, rounds.get(), stream.get());
         SSV_LAUNCH_CHECK();
@@ -466,7 +505,7 @@ template <typename S>
 void Sweep<S>::run(S* out, const KState* st, int* err, cudaStream_t s) const {
     int bars = 0;  // levels of the longest chunk
     for (int c = 0; c < plan.nchunks; ++c) bars = std::max(bars, plan.chunk_lev[c + 1] - plan.chunk_lev[c]);
-    SweepArgs a{stream.get(), rounds.get(), round_ptr.get(), chunk_lev.get(), tx.get(), plan.nlev, plan.nchunks, bars,
+    SweepArgs a{stream.get(), rounds.get(), round_ptr.get(), chunk_lev.get(), tx.get(), plan.nchunks, bars,
                 plan.ctas, (plan.slots * (int)sizeof(S) + 127) / 128 * 128, plan.stage_bytes, stages, sweep_no_waits(), err};
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(plan.ctas);

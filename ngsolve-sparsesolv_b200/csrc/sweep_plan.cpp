@@ -58,7 +58,7 @@ bool SweepPlanHost::build(int n_, const int* rp, const int* ci, bool fwd, const 
     n = n_;
     nlev = (int)off.size() - 1;
     sbytes = sbytes_;
-    if (n <= 0 || nlev <= 0) return false;
+    if (n <= 0 || nlev <= 0 || ctas_max < 1) return false;
     ctas = pick_ctas(n, nlev, std::min(ctas_max, kSweepMaxCtas));
     const SweepCost& cost = sbytes > 8 ? kCostComplex : kCostReal;
     // the least it can take, from the widths alone: wide levels need no plan to be refused

@@ -64,7 +64,7 @@ struct SweepPlanHost {
     // Plans the sweep over the entries j < i (fwd) or j > i of the CSR pattern,
     // rows grouped by level (rows, off). `smem` = bytes for the window and
     // kSweepMinStages rounds, `stage` = most bytes of a round, ctas_max = largest
-    // cluster. False where a level does not fit the windows or a row a round, or where
+    // cluster (0: none). False where a level does not fit the windows or a row a round, or where
     // the sweep is estimated to take more than `worth` us, the time of the other way: at
     // most 16 of the SMs work, so wide levels are better launched one by one.
     bool build(int n, const int* rp, const int* ci, bool fwd, const std::vector<int>& rows,

@@ -129,6 +129,19 @@ int main() {
     expect("4 layers of 60000", layers(60000, 4, 3), 8, false);  // 43 / 40 against 10.7 / 10.5
     expect("diagonal", layers(1000, 1, 0), 8, false);        // 4.8 / 2.9 against 2.0 / 2.0
     expect("diagonal", layers(60000, 1, 0), 8, false);       // 13.8 / 11.8 against 2.2 / 2.1
+    // a device that places smaller clusters, or none
+    for (int most : {0, 1, 2, 8}) {
+        const Csr A = grid(20);
+        std::vector<int> lev, rows, off;
+        const int nl = build_levels(A.n, A.rp.data(), A.ci.data(), false, lev);
+        group_by_level(lev, nl, rows, off);
+        SweepPlanHost P;
+        const bool ok = P.build(A.n, A.rp.data(), A.ci.data(), true, rows, off, 8, 221000, 40960, most);
+        if (ok != (most > 0) || (ok && P.ctas > most)) {
+            std::printf("clusters of %d at most: built %d with %d\n", most, (int)ok, P.ctas);
+            ++fails;
+        }
+    }
     if (!fails) std::printf("ok\n");
     return fails ? 1 : 0;
 }

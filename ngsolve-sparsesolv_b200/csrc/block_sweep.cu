@@ -83,27 +83,37 @@ k_blk_sweep(int s0, int s1, const int* __restrict__ prow, const int* __restrict_
 }
 
 // An oversized block: its internal couplings (loc, lv: `width` columns of nr, padded with
-// 0 * slot nr) and level offsets go to shared memory before the wait, the couplings to
-// other blocks are folded into the right-hand side after it.
-template <typename S, typename SL, bool FWD>
+// 0 * slot nr; REST: then `rest` entries past the width, those of row q from rrp[q]) and level
+// offsets go to shared memory before the wait, the couplings to other blocks are folded into
+// the right-hand side after it.
+template <typename S, typename SL, bool FWD, bool REST>
 __global__ void __launch_bounds__(kBigThreads)
-k_big_sweep(int nlev, int nr, int width, const int* __restrict__ lev, const int* __restrict__ rows,
-            const int* __restrict__ loc, const SL* __restrict__ lv, const int* __restrict__ xrp,
-            const int* __restrict__ xcol, const SL* __restrict__ xv, const S* __restrict__ inv,
-            const S* __restrict__ x, const double* __restrict__ sc, S* y, const KState* st) {
+k_big_sweep(int nlev, int nr, int width, int rest, const int* __restrict__ lev, const int* __restrict__ rows,
+            const int* __restrict__ loc, const SL* __restrict__ lv, const int* __restrict__ rrp,
+            const int* __restrict__ xrp, const int* __restrict__ xcol, const SL* __restrict__ xv,
+            const S* __restrict__ inv, const S* __restrict__ x, const double* __restrict__ sc, S* y, const KState* st) {
     extern __shared__ __align__(16) unsigned char big_smem[];
     const int tid = threadIdx.x;
     const int qa = lev[0];
     S* ys = reinterpret_cast<S*>(big_smem);
     S* xs = ys + nr + 1;
     SL* sv = reinterpret_cast<SL*>(xs + nr + 1);
-    int* sl = reinterpret_cast<int*>(sv + (size_t)width * nr + (width * nr & 1));
-    int* slev = sl + width * nr;
-    for (int e = tid; e < width * nr; e += kBigThreads) {
+    const int pad = width * nr, all = pad + (REST ? rest : 0);
+    int* sl = reinterpret_cast<int*>(sv + all + (all & 1));
+    int* slev = sl + all;
+    int* srp = slev + nlev + 1;
+    for (int e = tid; e < all; e += kBigThreads) {
         sv[e] = lv[e];
         sl[e] = loc[e];
     }
     for (int l = tid; l <= nlev; l += kBigThreads) slev[l] = lev[l] - qa;
+    if constexpr (REST)
+        for (int q = tid; q <= nr; q += kBigThreads) srp[q] = pad + (q < nr ? rrp[qa + q] : rest);
+    auto past_width = [&](S a, int q) {
+        if constexpr (REST)
+            for (int e = srp[q]; e < srp[q + 1]; ++e) a = a - hi_of_any(sv[e]) * ys[sl[e]];
+        return a;
+    };
     if (tid == 0) ys[nr] = ST<S>::zero();
     pdl_gate();
     if (st && st->done) return;
@@ -143,12 +153,12 @@ k_big_sweep(int nlev, int nr, int width, const int* __restrict__ lev, const int*
             for (int u = 0; u < kBigWidth; ++u)
                 if (u < width) s = s - hi_of_any(w[u]) * g[u];
             for (int u = kBigWidth; u < width; ++u) s = s - hi_of_any(sv[u * nr + q]) * ys[sl[u * nr + q]];
-            ys[q] = s;
+            ys[q] = past_width(s, q);
         }
         for (int p = slev[l] + tid + kBigThreads; p < slev[l + 1]; p += kBigThreads) {
             S a = xs[p];
             for (int u = 0; u < width; ++u) a = a - hi_of_any(sv[u * nr + p]) * ys[sl[u * nr + p]];
-            ys[p] = a;
+            ys[p] = past_width(a, p);
         }
         if (l + 1 < nlev) operands(l + 1);
         __syncthreads();
@@ -157,9 +167,10 @@ k_big_sweep(int nlev, int nr, int width, const int* __restrict__ lev, const int*
 }
 
 template <typename S, typename SL>
-static size_t big_bytes(int nr, int width, int nlev) {
-    return 2 * (size_t)(nr + 1) * sizeof(S) + ((size_t)width * nr + 1) * sizeof(SL) + (size_t)width * nr * 4 +
-           (size_t)(nlev + 1) * 4 + 16;
+static size_t big_bytes(int nr, int width, size_t rest, int nlev) {
+    const size_t all = (size_t)width * nr + rest;
+    return 2 * (size_t)(nr + 1) * sizeof(S) + (all + 1) * sizeof(SL) + all * 4 + (size_t)(nlev + 1) * 4 +
+           (rest > 0 ? (size_t)(nr + 1) * 4 : 0) + 16;
 }
 
 // coefficients of the slices: forward L_ij / L_ii, backward L_ji * (1 / L_ii)
@@ -196,8 +207,9 @@ __global__ void k_blk_fill(int slices, int lanes, int fwd, const int* __restrict
 
 // coefficients of an oversized block's rows q of rows[qa ..]
 template <typename S, typename SO>
-__global__ void k_big_fill(int nr, int qa, int width, int fwd, const int* __restrict__ rows,
-                           const int* __restrict__ lsrc, const int* __restrict__ xrp, const int* __restrict__ xsrc,
+__global__ void k_big_fill(int nr, int qa, int width, int rest, int fwd, const int* __restrict__ rows,
+                           const int* __restrict__ lsrc, const int* __restrict__ rrp, const int* __restrict__ xrp,
+                           const int* __restrict__ xsrc,
                            const int* __restrict__ Lrp, const S* __restrict__ Lv, const S* __restrict__ inv,
                            SO* __restrict__ lv, SO* __restrict__ xv) {
     auto put = [](S x) {
@@ -212,6 +224,9 @@ __global__ void k_big_fill(int nr, int qa, int width, int fwd, const int* __rest
             return put(fwd ? ST<S>::div(Lv[k], d) : Lv[k] * w);
         };
         for (int u = 0; u < width; ++u) lv[u * nr + q] = scaled(lsrc[u * nr + q]);
+        if (rest > 0)
+            for (int e = rrp[qa + q]; e < (q + 1 < nr ? rrp[qa + q + 1] : rest); ++e)
+                lv[width * nr + e] = scaled(lsrc[width * nr + e]);
         for (int e = xrp[qa + q]; e < xrp[qa + q + 1]; ++e) xv[e] = scaled(xsrc[e]);
     }
 }
@@ -242,7 +257,7 @@ void BlockSweep<S>::build(int lanes_, const std::vector<int>& boff, const std::v
     int smem_optin = 0;
     SSV_CUDA(cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, 0));
     struct Layout {
-        std::vector<int> off, col, src, isrc, xrp, xcol, xsrc, loc, lsrc;
+        std::vector<int> off, col, src, isrc, rrp, xrp, xcol, xsrc, loc, lsrc;
         int big_max = 0;
     } lay[2];
     auto direction = [&](bool fwd, Dir& D, Layout& h, const std::vector<Run>& runs, const std::vector<int>& rows,
@@ -294,6 +309,7 @@ void BlockSweep<S>::build(int lanes_, const std::vector<int>& boff, const std::v
         }
         // oversized blocks
         xrp.assign(rows.size() + 1, 0);
+        h.rrp.assign(rows.size(), 0);
         std::vector<int> at(n > 0 && !rows.empty() ? n : 0, -1);
         D.steps.clear();
         for (const Run& q : runs) {
@@ -304,36 +320,58 @@ void BlockSweep<S>::build(int lanes_, const std::vector<int>& boff, const std::v
             } else {
                 const int qa = lv[q.a], qb = lv[q.b], nr = qb - qa;
                 for (int p = qa; p < qb; ++p) at[rows[p]] = p - qa;
-                int width = 0;
-                for (int p = qa; p < qb; ++p) {
-                    int c = 0;
-                    for (int k = e0(rows[p]); k < e1(rows[p]); ++k) c += at[ci[k]] >= 0;
-                    width = std::max(width, c);
+                std::vector<int> has(nr, 0);  // internal entries of each row
+                for (int p = qa; p < qb; ++p)
+                    for (int k = e0(rows[p]); k < e1(rows[p]); ++k) has[p - qa] += at[ci[k]] >= 0;
+                int width = nr > 0 ? *std::max_element(has.begin(), has.end()) : 0;
+                size_t rest = 0;
+                auto fits = [&] { return big_bytes<S, S>(nr, width, rest, q.b - q.a) + 1024 <= (size_t)smem_optin; };
+                if (!fits()) {  // a few long rows: the width that takes the fewest entries in all
+                    std::vector<int> by = has;
+                    std::sort(by.begin(), by.end());
+                    size_t past = 0, least = ~size_t(0);  // entries past the width by[t]
+                    for (int t = nr - 1; t >= 0; --t) {
+                        if (t + 1 < nr) past += (size_t)(nr - 1 - t) * (by[t + 1] - by[t]);
+                        if ((size_t)by[t] * nr + past < least) {
+                            least = (size_t)by[t] * nr + past;
+                            width = by[t];
+                            rest = past;
+                        }
+                    }
                 }
                 st.qa = qa;
                 st.nr = nr;
-                st.width = width;
-                st.base = (int)loc.size();
-                loc.resize(st.base + (size_t)width * nr, nr);
-                lsrc.resize(st.base + (size_t)width * nr, -1);
+                if (fits()) {
+                    st.smem = (int)big_bytes<S, S>(nr, width, rest, q.b - q.a);
+                    st.width = width;
+                    st.rest = (int)rest;
+                    st.base = (int)loc.size();
+                    const size_t pad = st.base + (size_t)width * nr;
+                    loc.resize(pad, nr);
+                    lsrc.resize(pad, -1);
+                }
                 for (int p = qa; p < qb; ++p) {
                     int c = 0;
-                    for (int k = e0(rows[p]); k < e1(rows[p]); ++k) {
-                        const int a = at[ci[k]];
-                        if (a >= 0) {
-                            loc[st.base + (size_t)c * nr + p - qa] = a;
-                            lsrc[st.base + (size_t)c * nr + p - qa] = from(k);
-                            ++c;
-                        } else {
-                            xcol.push_back(ci[k]);
-                            xsrc.push_back(from(k));
+                    if (st.smem > 0) {
+                        h.rrp[p] = (int)(loc.size() - st.base - (size_t)width * nr);
+                        for (int k = e0(rows[p]); k < e1(rows[p]); ++k) {
+                            const int a = at[ci[k]];
+                            if (a < 0) {
+                                xcol.push_back(ci[k]);
+                                xsrc.push_back(from(k));
+                            } else if (c < width) {
+                                loc[st.base + (size_t)c * nr + p - qa] = a;
+                                lsrc[st.base + (size_t)c * nr + p - qa] = from(k);
+                                ++c;
+                            } else {
+                                loc.push_back(a);
+                                lsrc.push_back(from(k));
+                            }
                         }
                     }
                     xrp[p + 1] = (int)xcol.size();
                 }
                 for (int p = qa; p < qb; ++p) at[rows[p]] = -1;
-                const size_t bytes = big_bytes<S, S>(nr, width, q.b - q.a);
-                st.smem = bytes + 1024 <= (size_t)smem_optin ? (int)bytes : 0;
                 h.big_max = std::max(h.big_max, st.smem);
             }
             D.steps.push_back(st);
@@ -352,7 +390,7 @@ void BlockSweep<S>::build(int lanes_, const std::vector<int>& boff, const std::v
         const Layout& h = lay[t];
         up(D.off, h.off); up(D.col, h.col); up(D.src, h.src); up(D.isrc, h.isrc);
         up(D.lev, t == 0 ? lev_f : lev_b); up(D.rows, t == 0 ? rows_f : rows_b);
-        up(D.loc, h.loc); up(D.lsrc, h.lsrc); up(D.xrp, h.xrp); up(D.xcol, h.xcol); up(D.xsrc, h.xsrc);
+        up(D.loc, h.loc); up(D.lsrc, h.lsrc); up(D.rrp, h.rrp); up(D.xrp, h.xrp); up(D.xcol, h.xcol); up(D.xsrc, h.xsrc);
     }
     const int big_max = std::max(lay[0].big_max, lay[1].big_max);
     if (h_prow.empty()) prow.release();
@@ -361,10 +399,10 @@ void BlockSweep<S>::build(int lanes_, const std::vector<int>& boff, const std::v
     SSV_CUDA(cudaStreamSynchronize(s));
     if (big_max > 0) {
         const auto kind = cudaFuncAttributeMaxDynamicSharedMemorySize;
-        SSV_CUDA(cudaFuncSetAttribute(k_big_sweep<S, S, true>, kind, smem_optin - 1024));
-        SSV_CUDA(cudaFuncSetAttribute(k_big_sweep<S, S, false>, kind, smem_optin - 1024));
-        SSV_CUDA(cudaFuncSetAttribute(k_big_sweep<S, SL, true>, kind, smem_optin - 1024));
-        SSV_CUDA(cudaFuncSetAttribute(k_big_sweep<S, SL, false>, kind, smem_optin - 1024));
+        auto allow = [&](auto... k) { (SSV_CUDA(cudaFuncSetAttribute(k, kind, smem_optin - 1024)), ...); };
+        allow(k_big_sweep<S, S, true, false>, k_big_sweep<S, S, false, false>, k_big_sweep<S, SL, true, false>,
+              k_big_sweep<S, SL, false, false>, k_big_sweep<S, S, true, true>, k_big_sweep<S, S, false, true>,
+              k_big_sweep<S, SL, true, true>, k_big_sweep<S, SL, false, true>);
     }
 }
 
@@ -385,7 +423,7 @@ void BlockSweep<S>::fill(bool lo_, cudaStream_t s) {
             for (const Step& q : D.steps)
                 if (q.kind == 2 && q.smem > 0)
                     k_big_fill<S><<<grid_for(q.nr, 128), 128, 0, s>>>(
-                        q.nr, q.qa, q.width, fwd, D.rows.get(), D.lsrc.get() + q.base, D.xrp.get(),
+                        q.nr, q.qa, q.width, q.rest, fwd, D.rows.get(), D.lsrc.get() + q.base, D.rrp.get(), D.xrp.get(),
                         D.xsrc.get(), Lrp, Lv, inv, lv.get() + q.base, xv.get());
             SSV_LAUNCH_CHECK();
         };
@@ -430,8 +468,9 @@ static void run_blocks(const BlockSweep<S>& w, const typename BlockSweep<S>::Dir
                 default: go(std::integral_constant<int, 32>()); break;
             }
         } else if (q.smem > 0) {
-            launch_big(k_big_sweep<S, SL, FWD>, q.smem, s, q.b - q.a, q.nr, q.width, D.lev.get() + q.a, D.rows.get(),
-                       D.loc.get() + q.base, lv + q.base, D.xrp.get(), D.xcol.get(), xv, w.inv, x, sc, y, st);
+            launch_big(q.rest > 0 ? k_big_sweep<S, SL, FWD, true> : k_big_sweep<S, SL, FWD, false>, q.smem, s, q.b - q.a,
+                       q.nr, q.width, q.rest, D.lev.get() + q.a, D.rows.get(), D.loc.get() + q.base, lv + q.base,
+                       D.rrp.get(), D.xrp.get(), D.xcol.get(), xv, w.inv, x, sc, y, st);
         } else if (FWD) {
             launch_k(k_ic_fwd_cta<S, SL>, 1, 256, s, q.b - q.a, D.lev.get() + q.a, D.rows.get(), w.Lrp, w.Lci, full, x,
                      sc, y, st);

@@ -14,7 +14,9 @@
 //     sums and resolves the block's own couplings by shuffles after that;
 //   - an oversized block is staged in shared memory the same way, and its level
 //     sets are swept by one CTA with the next level's operands already in
-//     registers at each barrier.
+//     registers at each barrier. Rows are padded to the longest one where that
+//     fits, else to the width that takes the least, the rest of a row following
+//     row by row; a block that does not fit at all keeps its CSR rows.
 #pragma once
 
 #include <vector>
@@ -32,7 +34,8 @@ struct BlockSweep {
     // staged in smem bytes (0: too large, swept from the CSR factor)
     struct Step {
         int kind, a, b;
-        int smem = 0, qa = 0, nr = 0, width = 0, base = 0;  // first row of the list, rows, internal entries a row
+        // first row of the list, rows, internal entries a row, entries past them, first of all these
+        int smem = 0, qa = 0, nr = 0, width = 0, rest = 0, base = 0;
     };
     // one run of blocks or one oversized block, in processing order
     struct Run {
@@ -44,7 +47,7 @@ struct BlockSweep {
         DevBuf<S> v, iv;
         DevBuf<SL> v_lo, iv_lo;
         DevBuf<int> lev, rows;            // oversized blocks: level offsets, rows by level
-        DevBuf<int> loc, lsrc, xrp, xcol, xsrc;
+        DevBuf<int> loc, lsrc, rrp, xrp, xcol, xsrc;  // rrp: a row's entries past the width, by row of the list
         DevBuf<S> lv, xv;
         DevBuf<SL> lv_lo, xv_lo;
     };

@@ -278,23 +278,23 @@ void run_mrtr(ssv_solver* sv, const ssv_config& cfg, const S* d_b, S* d_x, ssv_r
     }
     MrtrPattern<S>& P = mrtr_of<S>(sv);
     if (!P.built) {
-        std::vector<int> lrp, lci, lsrc, urp, uci, usrc, lev, rws, off;
+        std::vector<int> lrp, lci, lsrc, urp, uci, usrc, lev, rws_f, off_f, rws_b, off_b;
         lower_pattern(n, A->h_rp.data(), A->h_ci.data(), lrp, lci, lsrc);
         transpose_pattern(n, lrp, lci, urp, uci, usrc);
         P.fwd.clear();
         P.bwd.clear();
         int nl = build_levels(n, lrp.data(), lci.data(), false, lev);
-        group_by_level(lev, nl, rws, off);
-        P.rows_f.upload(rws.data(), rws.size(), s);
-        for (int l = 0; l < nl; ++l) P.fwd.push_back({off[l], off[l + 1]});
+        group_by_level(lev, nl, rws_f, off_f);
+        P.rows_f.upload(rws_f.data(), rws_f.size(), s);
+        for (int l = 0; l < nl; ++l) P.fwd.push_back({off_f[l], off_f[l + 1]});
         P.diag = true;
         for (int i = 0; i < n && P.diag; ++i) P.diag = lrp[i] < lrp[i + 1] && lci[lrp[i + 1] - 1] == i;
-        if (P.diag) P.sweep_f.build(n, lrp, lci, true, rws, off, s);
         nl = build_levels(n, urp.data(), uci.data(), true, lev);
-        group_by_level(lev, nl, rws, off);
-        P.rows_b.upload(rws.data(), rws.size(), s);
-        for (int l = 0; l < nl; ++l) P.bwd.push_back({off[l], off[l + 1]});
-        if (P.diag && P.sweep_f.ready) P.sweep_b.build(n, urp, uci, false, rws, off, s);
+        group_by_level(lev, nl, rws_b, off_b);
+        P.rows_b.upload(rws_b.data(), rws_b.size(), s);
+        for (int l = 0; l < nl; ++l) P.bwd.push_back({off_b[l], off_b[l + 1]});
+        if (P.diag)
+            build_sweeps(P.sweep_f, P.sweep_b, {n, lrp, lci, true, rws_f, off_f}, {n, urp, uci, false, rws_b, off_b}, s);
         P.sweep_err.init(s);
         P.Lrp.upload(lrp.data(), lrp.size(), s);
         P.Lci.upload(lci.data(), lci.size(), s);

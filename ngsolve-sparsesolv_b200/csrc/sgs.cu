@@ -58,16 +58,15 @@ template <typename S> SgsDevice<S>& sgs_of(ssv_precond* p);
 template <> SgsDevice<double>& sgs_of<double>(ssv_precond* p) { return p->sgs_d; }
 template <> SgsDevice<zdouble>& sgs_of<zdouble>(ssv_precond* p) { return p->sgs_z; }
 
-template <typename S>
 static void levels_of(int n, const std::vector<int>& rp, const std::vector<int>& ci, bool upper,
-                      std::vector<std::pair<int, int>>& ranges, DevBuf<int>& rows_d, Sweep<S>& sweep, cudaStream_t s) {
-    std::vector<int> lev, rows, off;
+                      std::vector<std::pair<int, int>>& ranges, DevBuf<int>& rows_d, std::vector<int>& rows,
+                      std::vector<int>& off, cudaStream_t s) {
+    std::vector<int> lev;
     const int nl = build_levels(n, rp.data(), ci.data(), upper, lev);
     group_by_level(lev, nl, rows, off);
     ranges.clear();
     for (int l = 0; l < nl; ++l) ranges.push_back({off[l], off[l + 1]});
     rows_d.upload(rows.data(), rows.size(), s);
-    sweep.build(n, rp, ci, !upper, rows, off, s);
 }
 
 template <typename S>
@@ -92,8 +91,11 @@ static void sgs_update_t(ssv_precond* p) {
         vals = reinterpret_cast<const S*>(p->vals_bc.get());
     }
     if (!g.built) {
-        levels_of(n, A->h_rp, A->h_ci, false, g.fwd_lev, g.rows_f, g.sweep_f, s);
-        levels_of(n, A->h_rp, A->h_ci, true, g.bwd_lev, g.rows_b, g.sweep_b, s);
+        std::vector<int> rws_f, off_f, rws_b, off_b;
+        levels_of(n, A->h_rp, A->h_ci, false, g.fwd_lev, g.rows_f, rws_f, off_f, s);
+        levels_of(n, A->h_rp, A->h_ci, true, g.bwd_lev, g.rows_b, rws_b, off_b, s);
+        build_sweeps(g.sweep_f, g.sweep_b, {n, A->h_rp, A->h_ci, true, rws_f, off_f},
+                     {n, A->h_rp, A->h_ci, false, rws_b, off_b}, s);
         g.sweep_err.init(s);
         g.inv.alloc(n);
         g.tmp.alloc(n);

@@ -214,17 +214,16 @@ void ICDevice<S>::build_pattern(int n_, const std::vector<int>& rp, const std::v
     }
     transpose_pattern(n, lrp, lci, urp, uci, usrc);
     if (!abmc) {
-        std::vector<int> lev, rws, off;
+        std::vector<int> lev, rws_f, off_f, rws_b, off_b;
         num_levels_f = build_levels(n, lrp.data(), lci.data(), false, lev);
-        group_by_level(lev, num_levels_f, rws, off);
-        rows_f.upload(rws.data(), rws.size(), s);
-        for (int l = 0; l < num_levels_f; ++l) fwd_launch.push_back({off[l], off[l + 1]});
-        sweep_f.build(n, lrp, lci, true, rws, off, s);
+        group_by_level(lev, num_levels_f, rws_f, off_f);
+        rows_f.upload(rws_f.data(), rws_f.size(), s);
+        for (int l = 0; l < num_levels_f; ++l) fwd_launch.push_back({off_f[l], off_f[l + 1]});
         num_levels_b = build_levels(n, urp.data(), uci.data(), true, lev);
-        group_by_level(lev, num_levels_b, rws, off);
-        rows_b.upload(rws.data(), rws.size(), s);
-        for (int l = 0; l < num_levels_b; ++l) bwd_launch.push_back({off[l], off[l + 1]});
-        if (sweep_f.ready) sweep_b.build(n, urp, uci, false, rws, off, s);
+        group_by_level(lev, num_levels_b, rws_b, off_b);
+        rows_b.upload(rws_b.data(), rws_b.size(), s);
+        for (int l = 0; l < num_levels_b; ++l) bwd_launch.push_back({off_b[l], off_b[l + 1]});
+        build_sweeps(sweep_f, sweep_b, {n, lrp, lci, true, rws_f, off_f}, {n, urp, uci, false, rws_b, off_b}, s);
     }
     // missing diagonal (ic_preconditioner.hpp:1221-1226 / :1358-1363): first
     // row in processing order whose last lower entry is not the diagonal
@@ -327,13 +326,14 @@ void ICDevice<S>::build_pattern(int n_, const std::vector<int>& rp, const std::v
         // 21.3 / 18.9 us, 41^3 29.1 / 25.8 against 27.2 / 23.8, 64^3 116 / 122 against 36 / 30;
         // complex, 12^3 18.3 / 16.5 against 20.6 / 17.0, 16^3 25.4 / 23.2 against 21.2 / 17.7.
         const double launches = 2.4 * (double)run_f.size();
-        std::vector<int> rws, off;
+        std::vector<int> rws_f, off_f, rws_b, off_b;
         const int nl = build_levels(n, lrp.data(), lci.data(), false, lev);
-        group_by_level(lev, nl, rws, off);
-        if (sweep_f.build(n, lrp, lci, true, rws, off, launches, s)) {
+        group_by_level(lev, nl, rws_f, off_f);
+        if (sweep_least_us(off_f, (int)sizeof(S)) <= launches) {
             const int nu = build_levels(n, urp.data(), uci.data(), true, lev);
-            group_by_level(lev, nu, rws, off);
-            sweep_b.build(n, urp, uci, false, rws, off, launches, s);
+            group_by_level(lev, nu, rws_b, off_b);
+            build_sweeps(sweep_f, sweep_b, {n, lrp, lci, true, rws_f, off_f, launches},
+                         {n, urp, uci, false, rws_b, off_b, launches}, s);
         }
         if (!swept())
             blocks.build(lanes_blk, bo, run_f, run_b, h_rows_f, h_lev_f, h_rows_b, h_lev_b, lrp, lci, urp, uci, usrc, s);

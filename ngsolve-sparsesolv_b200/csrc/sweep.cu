@@ -1,8 +1,11 @@
 // sweep.cu -- see sweep.cuh.
+#include "host_threads.hpp"
 #include "objects.cuh"
 #include "sweep.cuh"
 
 #include <atomic>
+#include <cstring>
+#include <type_traits>
 
 namespace ssv {
 
@@ -21,6 +24,10 @@ constexpr int kWaitTries = 1 << 18;
 static std::atomic<bool> g_no_waits{false};
 bool sweep_no_waits() { return g_no_waits; }
 void set_sweep_wait(int tries) { g_no_waits = tries == 0; }
+
+// rows from which on the plans of the two directions are made on two host threads (50 ns a row
+// each, a thread some 30 us)
+constexpr int kSideBySide = 2000;
 
 struct SweepArgs {
     const unsigned char* stream;
@@ -436,32 +443,82 @@ static int placeable_ctas() {
 }
 
 template <typename S>
-bool Sweep<S>::build(int n, const std::vector<int>& rp, const std::vector<int>& ci, bool fwd_,
-                     const std::vector<int>& rows, const std::vector<int>& off, double worth, cudaStream_t s) {
-    ready = false;
-    fwd = fwd_;
-    if (!plan.build(n, rp.data(), ci.data(), fwd, rows, off, (int)sizeof(S), kSmemBytes - kBarBytes, kStageBytes,
-                    placeable_ctas<S>(), worth)) {
+bool Sweep<S>::plan_host(const SweepRows& q, int ctas_max) {
+    const double worth = q.worth >= 0.0 ? q.worth : level_launches_us(q.n, q.rp.data(), q.rows, q.off, (int)sizeof(S));
+    if (!plan.build(q.n, q.rp.data(), q.ci.data(), q.fwd, q.rows, q.off, (int)sizeof(S), kSmemBytes - kBarBytes, kStageBytes,
+                    ctas_max, worth)) {
         plan = SweepPlanHost();
         return false;
     }
-    rowpos.upload(plan.rowpos.data(), plan.rowpos.size(), s);
-    pos.upload(plan.pos.data(), plan.pos.size(), s);
-    lev.upload(plan.lev.data(), plan.lev.size(), s);
-    cta.upload(plan.cta.data(), plan.cta.size(), s);
-    tgt_ptr.upload(plan.tgt_ptr.data(), plan.tgt_ptr.size(), s);
-    tgt.upload(plan.tgt.data(), plan.tgt.size(), s);
-    slice_round.upload(plan.slice_round.data(), plan.slice_round.size(), s);
-    slice_chunk0.upload(plan.slice_chunk0.data(), plan.slice_chunk0.size(), s);
-    round_ptr.upload(plan.round_ptr.data(), plan.round_ptr.size(), s);
-    chunk_lev.upload(plan.chunk_lev.data(), plan.chunk_lev.size(), s);
-    tx.upload(plan.tx.data(), plan.tx.size(), s);
-    xs.alloc(plan.rowpos.size());
-    xs.zero(s);
-    stages = 0;  // laid out by the first fill()
-    SSV_CUDA(cudaStreamSynchronize(s));
-    ready = true;
+    // the lists side by side, as they lie on the device; only the kernels need them from here on
+    places.clear();
+    size_t at = 0;
+    auto room = [&](size_t bytes) {
+        places.push_back(at);
+        at += (bytes + 255) / 256 * 256;
+    };
+    auto lists = [&](auto&& f) {
+        f(plan.rowpos); f(plan.pos); f(plan.lev); f(plan.tgt_ptr); f(plan.tgt); f(plan.slice_round); f(plan.slice_chunk0);
+        f(plan.round_ptr); f(plan.chunk_lev); f(plan.tx); f(plan.cta);
+    };
+    lists([&](auto& v) { room(v.size() * sizeof(v[0])); });
+    packed.resize(at);
+    size_t k = 0;
+    lists([&](auto& v) {
+        if (!v.empty()) std::memcpy(packed.data() + places[k], v.data(), v.size() * sizeof(v[0]));
+        ++k;
+    });
+    room(plan.rounds.size() * sizeof(SweepRound));
+    room(plan.slice_off16.size() * sizeof(int));
+    room(plan.rowpos.size() * sizeof(S));
+    room(plan.stream_bytes);  // (the FP32 form takes less)
+    places.push_back(at);
+    auto drop = [](auto& v) { std::remove_reference_t<decltype(v)>().swap(v); };
+    drop(plan.rowpos); drop(plan.pos); drop(plan.lev); drop(plan.tgt_ptr); drop(plan.tgt); drop(plan.slice_round);
+    drop(plan.slice_chunk0); drop(plan.tx); drop(plan.cta);
     return true;
+}
+
+template <typename S>
+void build_sweeps(Sweep<S>& f, Sweep<S>& b, const SweepRows& qf, const SweepRows& qb, cudaStream_t s) {
+    f.ready = b.ready = false;
+    f.fwd = qf.fwd;
+    b.fwd = qb.fwd;
+    const int ctas = placeable_ctas<S>();
+    bool ok[2] = {false, false};
+    auto one = [&](int t) { ok[t] = t == 0 ? f.plan_host(qf, ctas) : b.plan_host(qb, ctas); };
+    if (qf.n >= kSideBySide) {
+        run_threads(2, one);
+    } else {
+        one(0);
+        if (ok[0]) one(1);
+    }
+    if (!ok[0] || !ok[1]) {
+        f.plan = b.plan = SweepPlanHost();
+        std::vector<unsigned char>().swap(f.packed);
+        std::vector<unsigned char>().swap(b.packed);
+        return;
+    }
+    f.mem.alloc(f.places.back() + b.places.back());
+    f.upload(f.mem.get(), s);
+    b.upload(f.mem.get() + f.places.back(), s);
+    SSV_CUDA(cudaStreamSynchronize(s));
+    std::vector<unsigned char>().swap(f.packed);
+    std::vector<unsigned char>().swap(b.packed);
+    f.ready = b.ready = true;
+}
+
+template <typename S>
+void Sweep<S>::upload(unsigned char* at, cudaStream_t s) {
+    size_t k = 0;
+    auto set = [&](auto& v) {
+        v.p = reinterpret_cast<decltype(v.p)>(at + places[k++]);
+    };
+    set(rowpos); set(pos); set(lev); set(tgt_ptr); set(tgt); set(slice_round); set(slice_chunk0); set(round_ptr);
+    set(chunk_lev); set(tx); set(cta); set(rounds); set(slice_off16); set(xs); set(stream);
+    h2d_staged(at, packed.data(), packed.size(), s);
+    SSV_CUDA(cudaMemsetAsync(xs.get(), 0, sizeof(S) * (size_t)positions(), s));
+    stages = 0;  // laid out by the first fill()
 }
 
 template <typename S>
@@ -472,9 +529,11 @@ void Sweep<S>::fill(SweepOp op, const int* rp, const int* ci, const S* v, int dm
         lo = lo_;
         stages = 0;
         plan.layout((int)(lo ? sizeof(SLo) : sizeof(S)));  // FP32 rounds are no larger than the planned ones
-        stream.alloc(plan.stream_bytes);
-        rounds.upload(plan.rounds.data(), plan.rounds.size(), s);
-        slice_off16.upload(plan.slice_off16.data(), plan.slice_off16.size(), s);
+        auto put = [&](void* d, const void* h, size_t bytes) {
+            SSV_CUDA(cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, s));
+        };
+        put(rounds.get(), plan.rounds.data(), plan.rounds.size() * sizeof(SweepRound));
+        put(slice_off16.get(), plan.slice_off16.data(), plan.slice_off16.size() * sizeof(int));
         const int wb = (plan.slots * (int)sizeof(S) + 127) / 128 * 128;
         const int st = plan.ring_stages(kSmemBytes - wb - kBarBytes);
         smem = wb + st * plan.stage_bytes + kBarBytes;
@@ -546,5 +605,7 @@ void SweepFlag::check(cudaStream_t s) const {
 
 template struct Sweep<double>;
 template struct Sweep<zdouble>;
+template void build_sweeps(Sweep<double>&, Sweep<double>&, const SweepRows&, const SweepRows&, cudaStream_t);
+template void build_sweeps(Sweep<zdouble>&, Sweep<zdouble>&, const SweepRows&, const SweepRows&, cudaStream_t);
 
 }  // namespace ssv

@@ -52,6 +52,17 @@ struct SweepFlag {
     void check(cudaStream_t s) const;
 };
 
+// One direction's rows: the triangular part of a CSR pattern (entries j < i, or j > i, of every
+// row), the rows by level, and the time in us of the other way to sweep it (< 0: a launch per
+// level).
+struct SweepRows {
+    int n;
+    const std::vector<int>&rp, &ci;
+    bool fwd;
+    const std::vector<int>&rows, &off;
+    double worth = -1.0;
+};
+
 template <typename S>
 struct Sweep {
     SweepPlanHost plan;
@@ -59,23 +70,25 @@ struct Sweep {
     bool fwd = true;
     int stages = 0, smem = 0;
     bool lo = false;
-    DevBuf<unsigned char> stream;
-    DevBuf<int> rowpos, pos, lev, tgt_ptr, tgt, slice_round, slice_chunk0, slice_off16, round_ptr, chunk_lev;
-    DevBuf<uint8_t> cta;
-    DevBuf<uint32_t> tx;
-    DevBuf<SweepRound> rounds;
-    DevBuf<S> xs;  // inputs by position
+    // One allocation, the forward sweep's, holds the plans' lists, the rounds, the inputs by
+    // position (xs) and the streams of both directions: 28 took 2 ms at 30,000 rows, one 0.5.
+    DevBuf<unsigned char> mem;
+    std::vector<size_t> places;  // byte offsets of the parts, their size at the end
+    std::vector<unsigned char> packed;
+    template <typename T>
+    struct Part {
+        T* p = nullptr;
+        T* get() const { return p; }
+    };
+    Part<unsigned char> stream;
+    Part<int> rowpos, pos, lev, tgt_ptr, tgt, slice_round, slice_chunk0, slice_off16, round_ptr, chunk_lev;
+    Part<uint8_t> cta;
+    Part<uint32_t> tx;
+    Part<SweepRound> rounds;
+    Part<S> xs;
 
-    // Plans the sweep for a triangular part of the pattern (entries j < i or
-    // j > i of every row); false (and ready = false) where it does not fit or is
-    // estimated to take more than `worth` us, the time of the caller's other way.
-    bool build(int n, const std::vector<int>& rp, const std::vector<int>& ci, bool fwd, const std::vector<int>& rows,
-               const std::vector<int>& off, double worth, cudaStream_t s);
-    // The same against a launch per level.
-    bool build(int n, const std::vector<int>& rp, const std::vector<int>& ci, bool fwd, const std::vector<int>& rows,
-               const std::vector<int>& off, cudaStream_t s) {
-        return build(n, rp, ci, fwd, rows, off, level_launches_us(n, rp.data(), rows, off, (int)sizeof(S)), s);
-    }
+    bool plan_host(const SweepRows& q, int ctas_max);
+    void upload(unsigned char* at, cudaStream_t s);
     // Writes the records from the CSR values: d from the row's last or first
     // entry or from darr; omap = output index of every row (null = the row).
     // lo_ stores the coefficients in the FP32 form.
@@ -88,5 +101,10 @@ struct Sweep {
     void run(S* out, const KState* st, int* err, cudaStream_t s) const;
     int positions() const { return plan.nslices * 32; }
 };
+
+// Plans both sweeps of an object. They stay not ready where one does not fit or is estimated to
+// take longer than the caller's other way.
+template <typename S>
+void build_sweeps(Sweep<S>& f, Sweep<S>& b, const SweepRows& qf, const SweepRows& qb, cudaStream_t s);
 
 }  // namespace ssv

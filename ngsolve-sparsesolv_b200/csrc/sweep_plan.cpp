@@ -53,6 +53,16 @@ double level_launches_us(int n, const int* rp, const std::vector<int>& rows, con
     return us;
 }
 
+double sweep_least_us(const std::vector<int>& off, int sbytes, int ctas) {
+    const SweepCost& cost = sbytes > 8 ? kCostComplex : kCostReal;
+    double us = kCostStart;
+    for (size_t l = 0; l + 1 < off.size(); ++l) {
+        const int sl = ((off[l + 1] - off[l] + 31) / 32 + ctas - 1) / ctas;
+        us += cost.round * ((sl + kSweepWarps - 1) / kSweepWarps) + cost.slice * sl;
+    }
+    return us;
+}
+
 bool SweepPlanHost::build(int n_, const int* rp, const int* ci, bool fwd, const std::vector<int>& rows,
                           const std::vector<int>& off, int sbytes_, int smem, int stage, int ctas_max, double worth) {
     n = n_;
@@ -61,12 +71,7 @@ bool SweepPlanHost::build(int n_, const int* rp, const int* ci, bool fwd, const 
     if (n <= 0 || nlev <= 0 || ctas_max < 1) return false;
     ctas = pick_ctas(n, nlev, std::min(ctas_max, kSweepMaxCtas));
     const SweepCost& cost = sbytes > 8 ? kCostComplex : kCostReal;
-    // the least it can take, from the widths alone: wide levels need no plan to be refused
-    us = kCostStart;
-    for (int l = 0; l < nlev; ++l) {
-        const int sl = ((off[l + 1] - off[l] + 31) / 32 + ctas - 1) / ctas;
-        us += cost.round * ((sl + kSweepWarps - 1) / kSweepWarps) + cost.slice * sl;
-    }
+    us = sweep_least_us(off, sbytes, ctas);
     if (us > worth) return false;
     // positions, owners, levels
     rowpos.clear();

@@ -86,6 +86,9 @@ struct SweepPlanHost {
     }
 };
 
+// The least that a sweep over levels of these offsets can take on so many CTAs, in us, from their
+// widths alone: wide levels need no plan to be refused.
+double sweep_least_us(const std::vector<int>& off, int sbytes, int ctas = kSweepMaxCtas);
 // Estimated time in us of the same sweep with a launch per level, a thread per row.
 double level_launches_us(int n, const int* rp, const std::vector<int>& rows, const std::vector<int>& off, int sbytes);
 

@@ -677,23 +677,23 @@ k_mv_pi_restrict(int n, const int* __restrict__ rp, const int* __restrict__ ci, 
 #pragma unroll
         for (int c = 0; c < W; ++c) ax[c] = ay[c] = az[c] = 0.0;
         while (j >= 0) {
-                double rr[W];
-                load_row<W>(r + (size_t)j * NV + c0, rr);
-                const double ux = vx, uy = vy, uz = vz;
-                if constexpr (kReadAhead<NV>) {
-                    k += E;
-                    entry();
-                }
+            double rr[W];
+            load_row<W>(r + (size_t)j * NV + c0, rr);
+            const double ux = vx, uy = vy, uz = vz;
+            if constexpr (kReadAhead<NV>) {
+                k += E;
+                entry();
+            }
 #pragma unroll
-                for (int c = 0; c < W; ++c) {
-                    ax[c] += ux * rr[c];
-                    ay[c] += uy * rr[c];
-                    az[c] += uz * rr[c];
-                }
-                if constexpr (!kReadAhead<NV>) {
-                    k += E;
-                    entry();
-                }
+            for (int c = 0; c < W; ++c) {
+                ax[c] += ux * rr[c];
+                ay[c] += uy * rr[c];
+                az[c] += uz * rr[c];
+            }
+            if constexpr (!kReadAhead<NV>) {
+                k += E;
+                entry();
+            }
         }
         if (row + (int)gridDim.x * rpb - lane_row < n) head(row + gridDim.x * rpb);
 #pragma unroll
@@ -759,25 +759,25 @@ k_mv_pi_prolong(int n, const int* __restrict__ rp, const int* __restrict__ ci, c
 #pragma unroll
         for (int c = 0; c < W; ++c) sx[c] = sy[c] = sz[c] = 0.0;
         while (j >= 0) {
-                TG vgx[W], vgy[W], vgz[W];
-                load_row<W>(gx + (size_t)j * NV + c0, vgx);
-                load_row<W>(gy + (size_t)j * NV + c0, vgy);
-                load_row<W>(gz + (size_t)j * NV + c0, vgz);
-                const double ux = vx, uy = vy, uz = vz;
-                if constexpr (kReadAhead<NV>) {
-                    k += E;
-                    entry();
-                }
+            TG vgx[W], vgy[W], vgz[W];
+            load_row<W>(gx + (size_t)j * NV + c0, vgx);
+            load_row<W>(gy + (size_t)j * NV + c0, vgy);
+            load_row<W>(gz + (size_t)j * NV + c0, vgz);
+            const double ux = vx, uy = vy, uz = vz;
+            if constexpr (kReadAhead<NV>) {
+                k += E;
+                entry();
+            }
 #pragma unroll
-                for (int c = 0; c < W; ++c) {
-                    sx[c] += ux * (double)vgx[c];
-                    sy[c] += uy * (double)vgy[c];
-                    sz[c] += uz * (double)vgz[c];
-                }
-                if constexpr (!kReadAhead<NV>) {
-                    k += E;
-                    entry();
-                }
+            for (int c = 0; c < W; ++c) {
+                sx[c] += ux * (double)vgx[c];
+                sy[c] += uy * (double)vgy[c];
+                sz[c] += uz * (double)vgz[c];
+            }
+            if constexpr (!kReadAhead<NV>) {
+                k += E;
+                entry();
+            }
         }
         if (row + (int)gridDim.x * rpb - lane_row < n) head(row + gridDim.x * rpb);
 #pragma unroll

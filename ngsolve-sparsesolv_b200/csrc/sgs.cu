@@ -4,9 +4,11 @@
 // rows identity, constrained columns zero), output zeroed on constrained DOFs.
 // Both sweeps run level set by level set (the reference's LevelSchedule built
 // from the full pattern, entries j < i forward and j > i backward), in one
-// launch each (sweep.cuh), or one launch per level with one thread per row
-// where a level or a row is too large for that; the arithmetic of a row is the
-// reference's, in its order.
+// launch each (sweep.cuh), or one launch per level with one thread per row where
+// that is faster or a level or a row is too large. Level by level the arithmetic
+// of a row is the reference's, in its order. The one-launch sweeps keep the
+// coefficients multiplied by 1/a_ii and sum a row's entries in another order
+// (those of earlier levels first, in two partial sums), which differs by rounding.
 #include "objects.cuh"
 #include "solver_api.hpp"
 

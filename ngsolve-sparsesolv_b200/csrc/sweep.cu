@@ -19,7 +19,7 @@ constexpr int kSweepThreads = (kComputeWarps + 1) * 32;
 // late entries and targets of a row that are in registers before its level is due
 constexpr int kAhead = 4;
 constexpr int kBarBytes = (2 * kMaxStages + kSweepMaxLevels + 2) * 8;
-// tries of a wait before it gives up (a try suspends for up to a microsecond or so)
+// tries of a wait before it gives up (a try suspends for up to 3.9 us: a second in all)
 constexpr int kWaitTries = 1 << 18;
 static std::atomic<bool> g_no_waits{false};
 bool sweep_no_waits() { return g_no_waits; }
@@ -66,8 +66,8 @@ __device__ __forceinline__ void bar_arrive(unsigned b) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(b) : "memory");
 }
 // Waits for the phase of the given parity; false after kWaitTries (a constant: a limit in a
-// register costs the sweep 5 %). CLUSTER: what other CTAs
-// wrote to global memory before they arrived is visible too.
+// register costs the sweep 5 %). CLUSTER: what other CTAs wrote to global memory before they
+// arrived is visible too.
 template <bool CLUSTER = false>
 __device__ __forceinline__ bool bar_try(unsigned b, unsigned parity) {
     unsigned ok;

@@ -2,14 +2,17 @@
 //
 // A sweep y_i = f(x_i, sum over j before i of a_ij y_j) is a chain of level
 // sets: 100 to 600 of them on nodal and edge-element matrices, a few hundred to
-// a few thousand rows each. One launch per level costs 2.4 - 3.0 us a level
-// whatever the level holds. Here one thread-block cluster (2 - 16 CTAs, by the
-// mean level width) walks all levels:
+// a few thousand rows each. One launch per level costs 2.3 - 6 us a level, little
+// of it by its width. Here one thread-block cluster (2 - 16 CTAs, by the mean
+// level width and what the device can place) walks all levels, 0.4 us a level
+// while it fills the cluster's rounds once (2048 real rows), in proportion
+// beyond. Wide, few or scattered levels keep their launches (SweepPlanHost). In it:
 //   - every CTA owns a part of each level; its rows' records (coefficients,
 //     columns, diagonal, output index) are one contiguous stream, and a
 //     producer warp moves it and the inputs, which lie in the same order, into
-//     a ring of shared-memory stages with bulk copies, ahead of the chain; four
-//     groups of four warps take the rounds in turn;
+//     a ring of 4 or 8 shared-memory stages with bulk copies, ahead of the
+//     chain; four groups of four warps take the rounds in turn, each with stages
+//     of its own;
 //   - a row's result goes to the shared-memory windows of exactly those CTAs
 //     that need it, by st.async, which also counts the bytes into the level's
 //     mbarrier there: no barrier over the cluster and no fence on the chain;
